@@ -13,18 +13,20 @@
 //
 //   1. form A column-major in the CTA's scratch slot (Gamma_r is pre-permuted to the same column-major
 //      compound layout once per request, so this is a coalesced stream plus a block-diagonal add);
-//   2. blocked right-looking LU with partial pivoting (panel width NB): the panel is factored column by
-//      column with the LAPACK pivot measure |re|+|im| and first-index ties (izamax), the panel's row
-//      interchanges are applied to the other columns, the U12 row block is solved against L11 from shared
-//      memory, and the trailing matrix is updated by a 64x64-tiled complex GEMM from shared memory;
+//   2. LU with partial pivoting, LAPACK's pivot measure |re|+|im| and first-index ties (izamax): in FP64 the Crout form
+//      of lu_dmma.cuh on the FP64 tensor pipe; in FP32 (lu_factor below) a right-looking form, panel width NB, the
+//      trailing matrix updated by a tiled complex GEMM from shared memory;
 //   3. the permuted selector right-hand side is solved by blocked forward and back substitution and
 //      written out divided by beta.
 //
-// The same LU core serves the FP64 drop-in (R = double) and the mixed form (R = float for the
-// factorisation, FP64 residuals and refinement; see bse_mixed below).
+// The mixed form factors in FP32 (FP64 residuals and refinement; see solve_item_mixed below); dense matrices beyond the
+// Crout form's size also take lu_factor.
 #include "bse_core.cuh"
+#include "lu_dmma.cuh"
 
 #include <stdio.h>
+
+#include <type_traits>
 
 namespace dga {
 
@@ -337,10 +339,12 @@ __device__ bool lu_factor(C* __restrict__ A, int N, int ld, int* __restrict__ pi
 // Solve (L U) Y = B in place for the n_rhs columns of Y (column-major, leading dimension N), with the LU
 // factors of lu_factor (unit lower L below the diagonal, U on and above).  Blocked by 32 rows: the diagonal
 // block is solved by one warp per right-hand side (lane = row, the solved value broadcast by shuffle), the
-// rest of the rows are updated from the block copy in shared memory.
+// rest of the rows are updated from the block copy in shared memory.  L11: the diagonal block, yb: [n_rhs][32] the
+// solved block, both in shared memory.
 // ----------------------------------------------------------------------------------------------
 template <typename C, typename CY, int NR>
-__device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y, BseSmem<C>& sm) {
+__device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y,
+                                 C (*__restrict__ L11)[BSE_NB + 1], CY* __restrict__ yb) {
   constexpr int n_rhs = NR;
   // factor elements a thread has in flight in the row updates: eight where each one feeds several right-hand
   // sides; with one to three the registers go to the factorisation around the solve instead
@@ -349,13 +353,12 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
   using RY = decltype(CY::x);
   const int tid = threadIdx.x, T = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
-  CY* yb = reinterpret_cast<CY*>(&sm.u.t.A12[0][0]);  // [n_rhs][32] solved block
   // forward: L z = b
   for (int b0 = 0; b0 < N; b0 += BSE_NB) {
     const int bn = min(BSE_NB, N - b0);
     for (int e = tid; e < bn * bn; e += T) {
       const int r = e % bn, c = e / bn;
-      sm.u.t.L11[r][c] = A[(size_t)(b0 + c) * ld + b0 + r];
+      L11[r][c] = A[(size_t)(b0 + c) * ld + b0 + r];
     }
     __syncthreads();
     for (int s = warp; s < n_rhs; s += nwarps) {
@@ -365,7 +368,7 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
         yr.x = __shfl_sync(0xffffffffu, y.x, r);
         yr.y = __shfl_sync(0xffffffffu, y.y, r);
         if (lane > r && lane < bn) {
-          const C l = sm.u.t.L11[lane][r];
+          const C l = L11[lane][r];
           cfms(y, cmake<CY>((RY)l.x, (RY)l.y), yr);
         }
       }
@@ -415,21 +418,21 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
     const int bn = min(BSE_NB, N - b0);
     for (int e = tid; e < bn * bn; e += T) {
       const int r = e % bn, c = e / bn;
-      sm.u.t.L11[r][c] = A[(size_t)(b0 + c) * ld + b0 + r];
+      L11[r][c] = A[(size_t)(b0 + c) * ld + b0 + r];
     }
     __syncthreads();
     for (int s = warp; s < n_rhs; s += nwarps) {
       CY y = lane < bn ? Y[(size_t)s * N + b0 + lane] : cmake<CY>(RY(0), RY(0));
       for (int r = bn - 1; r >= 0; --r) {
         if (lane == r) {
-          const C u = sm.u.t.L11[r][r];
+          const C u = L11[r][r];
           y = cdiv(y, cmake<CY>((RY)u.x, (RY)u.y));
         }
         CY yr;
         yr.x = __shfl_sync(0xffffffffu, y.x, r);
         yr.y = __shfl_sync(0xffffffffu, y.y, r);
         if (lane < r) {
-          const C u = sm.u.t.L11[lane][r];
+          const C u = L11[lane][r];
           cfms(y, cmake<CY>((RY)u.x, (RY)u.y), yr);
         }
       }
@@ -474,6 +477,30 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
   }
 }
 
+// perm[i] = the original row at position i after the interchanges in piv (both N ints in shared memory).  One warp looks
+// for the rows that moved, 32 at a time, and swaps those in order.
+__device__ void build_perm(int N, const int* __restrict__ piv, int* __restrict__ perm) {
+  const int tid = threadIdx.x, T = blockDim.x;
+  for (int i = tid; i < N; i += T) perm[i] = i;
+  __syncthreads();
+  if (tid < 32) {
+    for (int i0 = 0; i0 < N; i0 += 32) {
+      const int p = i0 + tid < N ? piv[i0 + tid] : i0 + tid;
+      unsigned moved = __ballot_sync(0xffffffffu, p != i0 + tid);
+      while (moved) {
+        const int b = __ffs(moved) - 1, q = __shfl_sync(0xffffffffu, p, b);
+        moved &= moved - 1;
+        if (tid == 0) {
+          const int t = perm[i0 + b];
+          perm[i0 + b] = perm[q];
+          perm[q] = t;
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // Y = P * S where S is the n2-column selector (S[j, s] = 1 if the orbital pair of row j is s) and P the
 // row permutation recorded in piv.  perm is shared scratch of N ints.
 template <typename CY>
@@ -481,19 +508,7 @@ __device__ void permuted_selector(CY* __restrict__ Y, int N, int nv, int n_rhs, 
                                   int* __restrict__ perm) {
   using RY = decltype(CY::x);
   const int tid = threadIdx.x, T = blockDim.x;
-  for (int i = tid; i < N; i += T) perm[i] = i;
-  __syncthreads();
-  if (tid == 0) {
-    for (int i = 0; i < N; ++i) {
-      const int p = piv[i];
-      if (p != i) {
-        int t = perm[i];
-        perm[i] = perm[p];
-        perm[p] = t;
-      }
-    }
-  }
-  __syncthreads();
+  build_perm(N, piv, perm);
   for (int e = tid; e < N * n_rhs; e += T) {
     const int i = e % N, s = e / N;
     Y[(size_t)s * N + i] = cmake<CY>((perm[i] / nv == s) ? RY(1) : RY(0), RY(0));
@@ -501,14 +516,46 @@ __device__ void permuted_selector(CY* __restrict__ Y, int N, int nv, int n_rhs, 
   __syncthreads();
 }
 
+// Shared memory of the FP64 kernels: the factorisation's and the solves' buffers are never live at the same time.  The
+// pivots and the permutation (N ints each) follow it.
+template <int NT>
+struct Fp64Smem {
+  union {
+    LuSmem<NT> lu;
+    struct {
+      double2 L11[BSE_NB][BSE_NB + 1];
+      double2 yb[MAX_RHS * BSE_NB];
+    } solve;
+  };
+  int flag;
+};
+
+// Threads of an FP64 CTA.  Each thread holds one row of a panel up to N = 64 and 128; from there a CTA of 128 threads is
+// the faster one up to about N = 350 (four CTAs an SM hide one another's panels: 9.7 against 11.3 ms for 3,552 factorisations
+// of N = 240), a CTA of 256 above (18.2 against 20.6 ms for 1,184 of N = 480; 27.0 against 39.5 ms for 592 of N = 720), and
+// 64 threads up to N = 64 (2.95 against 3.28 ms for 29,600 of N = 40).
+constexpr int fp64_threads(int N) { return N <= 64 ? 64 : N <= 352 ? 128 : 256; }
+constexpr int fp64_min_blocks(int NT) { return 512 / NT; }  // 128 registers a thread
+
 // ----------------------------------------------------------------------------------------------
 // One work item in FP64: form A, LU, selector solve, X = Y / beta into out (rows (p,nu), n2 columns).
 // Returns the item's status bits.  All threads of the CTA call it.
 // ----------------------------------------------------------------------------------------------
-template <typename Source, int NR>
-__device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int nv, double beta,
+// The right-hand-side count is chosen per item (n2 = 1, 4, 9 or 16), which keeps one copy of the factorisation per kernel.
+template <int NT>
+__device__ void lu_solve_n2(int n2, const double2* __restrict__ A, int N, double2* __restrict__ Y, Fp64Smem<NT>& sm) {
+  switch (n2) {
+    case 1: lu_solve_inplace<double2, double2, 1>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
+    case 4: lu_solve_inplace<double2, double2, 4>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
+    case 9: lu_solve_inplace<double2, double2, 9>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
+    default: lu_solve_inplace<double2, double2, 16>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
+  }
+}
+
+template <typename Source, int NT>
+__device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int n2, int nv, double beta,
                                double2* __restrict__ o, double2* __restrict__ A, double2* __restrict__ Y,
-                               BseSmem<double2>& sm, int* piv, int* perm) {
+                               Fp64Smem<NT>& sm, int* piv, int* perm) {
   const int tid = threadIdx.x, T = blockDim.x;
   // form A column by column; the (pair, nu) split of a thread's rows advances by T = q_T nv + r_T per step
   {
@@ -534,15 +581,15 @@ __device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int
     }
   }
   __syncthreads();
-  const bool singular = lu_factor<double2>(A, N, N, piv, sm);
-  permuted_selector<double2>(Y, N, nv, NR, piv, perm);
-  lu_solve_inplace<double2, double2, NR>(A, N, N, Y, sm);
+  const bool singular = lu_factor_dmma<NT>(A, N, N, piv, sm.lu);
+  permuted_selector<double2>(Y, N, nv, n2, piv, perm);
+  lu_solve_n2<NT>(n2, A, N, Y, sm);
   // X[i][s] = Y[i][s] / beta, finiteness check
   if (tid == 0) sm.flag = 0;
   __syncthreads();
   bool bad = false;
-  for (int e = tid; e < N * NR; e += T) {
-    const int i = e / NR, s = e % NR;
+  for (int e = tid; e < N * n2; e += T) {
+    const int i = e / n2, s = e - i * n2;
     double2 y = Y[(size_t)s * N + i];
     y.x = y.x / beta;
     y.y = y.y / beta;
@@ -557,15 +604,15 @@ __device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int
 }
 
 // FP64 kernel: one CTA per work item, persistent over the list.
-template <typename Source, int NR>
-__global__ void __launch_bounds__(BSE_THREADS, 3)
+template <typename Source, int NT>
+__global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     bse_solve_sum_fp64_kernel(Source src, const WorkItem* __restrict__ work, int n_items, int N, int n2,
                               int nv, int W, int Q, double beta, double2* __restrict__ out,
                               int* __restrict__ status, double2* __restrict__ scratch, size_t slot_elems,
                               int redo_only) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
-  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
+  Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
   int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
   double2* Y = A + (size_t)N * N;
@@ -574,7 +621,7 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
     if (redo_only && (status[item] & DGA_ITEM_REDO) == 0) continue;
     const WorkItem wi = work[item];
     double2* o = out + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * (size_t)N * n2;
-    const int st = solve_item_fp64<Source, NR>(src, wi, N, nv, beta, o, A, Y, sm, piv, perm);
+    const int st = solve_item_fp64<Source, NT>(src, wi, N, n2, nv, beta, o, A, Y, sm, piv, perm);
     if (threadIdx.x == 0 && status) status[item] = st;
   }
 }
@@ -628,8 +675,9 @@ __device__ int solve_item_mixed(const StructuredSource& src, const WorkItem& wi,
   }
   __syncthreads();
   const bool singular = lu_factor<float2>(A, N, N, piv, sm);
+  double2* yb = reinterpret_cast<double2*>(&sm.u.t.A12[0][0]);
   permuted_selector<double2>(Y, N, nv, NR, piv, perm);
-  lu_solve_inplace<float2, double2, NR>(A, N, N, Y, sm);
+  lu_solve_inplace<float2, double2, NR>(A, N, N, Y, sm.u.t.L11, yb);
   double prev = 0.0;
   for (int e = tid; e < N * NR; e += T) prev = fmax(prev, fmax(fabs(Y[e].x), fabs(Y[e].y)));
   prev = block_max(prev, sm.red_val);
@@ -638,7 +686,7 @@ __device__ int solve_item_mixed(const StructuredSource& src, const WorkItem& wi,
   for (; it < max_iter; ++it) {
     structured_residual_permuted<NR>(src, wi.ch, wi.q, wi.w, N, nv, Y, Rb, perm, colsum,
                                      reinterpret_cast<double2*>(&sm.u));
-    lu_solve_inplace<float2, double2, NR>(A, N, N, Rb, sm);
+    lu_solve_inplace<float2, double2, NR>(A, N, N, Rb, sm.u.t.L11, yb);
     double dmax = 0.0, ymax = 0.0;
     for (int e = tid; e < N * NR; e += T) {
       const double2 d = Rb[e];
@@ -710,103 +758,97 @@ __global__ void __launch_bounds__(BSE_THREADS, DGA_MIXED_MIN_BLOCKS)
 // descriptor carries the sizes, the resident inputs and the output.  The per-item body is the same as the
 // single-problem kernels.
 // ----------------------------------------------------------------------------------------------
-// One item of a batch: the problem's descriptor gives its sizes, inputs and output; returns the status bits.
-template <bool MIXED, int NR>
-__device__ __forceinline__ int multi_item(const dga_bse_problem& d, const MultiItem& mi, int n_max, int max_iter,
-                                          double tol, unsigned char* slot, unsigned char* smem_raw, int* it_out) {
-  {
-    struct {
-      StructuredSource src;
-      int N, n2, nv, W, Q;
-      double beta;
-      double2* out;
-    } pb;
-    pb.n2 = d.n_orb * d.n_orb;
-    pb.nv = 2 * d.niv;
-    pb.N = pb.n2 * pb.nv;
-    pb.W = d.niw_half;
-    pb.Q = d.n_q;
-    pb.beta = d.beta;
-    pb.out = (double2*)d.out;
-    pb.src.gamma_cm = (const double2*)d.gamma_cm;
-    pb.src.chi0_inv = (const double2*)d.chi0_inv;
-    pb.src.uv = (const double2*)d.uv;
-    pb.src.n2 = pb.n2;
-    pb.src.nv = pb.nv;
-    pb.src.W = pb.W;
-    pb.src.Q = pb.Q;
-    pb.src.inv_beta2 = d.inv_beta2;
-    const WorkItem wi{mi.ch, mi.q, mi.w};
-    double2* o = pb.out + (((size_t)wi.ch * pb.Q + wi.q) * pb.W + wi.w) * (size_t)pb.N * pb.n2;
-    int st = 0, it = 0;
-    if (MIXED) {
-      BseSmem<float2>& sm = *reinterpret_cast<BseSmem<float2>*>(smem_raw);
-      int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<float2>));
-      int* perm = piv + n_max;
-      double2* colsum = reinterpret_cast<double2*>(smem_raw + mixed_colsum_offset(n_max));
-      float2* A = reinterpret_cast<float2*>(slot);
-      double2* Y = reinterpret_cast<double2*>(slot + (((size_t)pb.N * pb.N * sizeof(float2) + 255) & ~(size_t)255));
-      double2* Rb = Y + (size_t)pb.N * pb.n2;
-      st = solve_item_mixed<NR>(pb.src, wi, pb.N, pb.nv, pb.beta, max_iter, tol, o, A, Y, Rb, sm, piv, perm, colsum, &it);
-    } else {
-      BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
-      int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
-      int* perm = piv + n_max;
-      double2* A = reinterpret_cast<double2*>(slot);
-      double2* Y = A + (size_t)pb.N * pb.N;
-      st = solve_item_fp64<StructuredSource, NR>(pb.src, wi, pb.N, pb.nv, pb.beta, o, A, Y, sm, piv, perm);
-    }
-    *it_out = it;
-    return st;
+// A batch item's problem, from its descriptor.
+struct MultiProblem {
+  StructuredSource src;
+  WorkItem wi;
+  int N, n2, nv;
+  double2* o;
+  __device__ __forceinline__ MultiProblem(const dga_bse_problem& d, const MultiItem& mi) : wi{mi.ch, mi.q, mi.w} {
+    n2 = d.n_orb * d.n_orb;
+    nv = 2 * d.niv;
+    N = n2 * nv;
+    src.gamma_cm = (const double2*)d.gamma_cm;
+    src.chi0_inv = (const double2*)d.chi0_inv;
+    src.uv = (const double2*)d.uv;
+    src.n2 = n2;
+    src.nv = nv;
+    src.W = d.niw_half;
+    src.Q = d.n_q;
+    src.inv_beta2 = d.inv_beta2;
+    o = (double2*)d.out + (((size_t)wi.ch * d.n_q + wi.q) * d.niw_half + wi.w) * (size_t)N * n2;
   }
-}
+};
 
-template <bool MIXED, int NR>
-__global__ void __launch_bounds__(BSE_THREADS, MIXED ? DGA_MIXED_MIN_BLOCKS : 3)
-    bse_multi_kernel(const dga_bse_problem* __restrict__ probs, const MultiItem* __restrict__ work, int n_items,
-                     int n_max, int max_iter, double tol, int* __restrict__ status, int* __restrict__ iters,
-                     unsigned char* __restrict__ scratch, size_t slot_bytes, int redo_only) {
+// FP64 batch; redo_only: the re-solve of the items a mixed launch flagged. Shared memory and the scratch slot are sized
+// for the largest problem of the launch.
+template <int NT>
+__global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
+    bse_multi_fp64_kernel(const dga_bse_problem* __restrict__ probs, const MultiItem* __restrict__ work, int n_items,
+                          int n_max, int* __restrict__ status, int* __restrict__ iters,
+                          unsigned char* __restrict__ scratch, size_t slot_bytes, int redo_only) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned char* slot = scratch + (size_t)blockIdx.x * slot_bytes;
+  Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
+  int* perm = piv + n_max;
+  double2* A = reinterpret_cast<double2*>(scratch + (size_t)blockIdx.x * slot_bytes);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     if (redo_only && (status[item] & DGA_ITEM_REDO) == 0) continue;
     const MultiItem mi = work[item];
     const dga_bse_problem d = probs[mi.prob];
-    int it = 0;
-    const int st = multi_item<MIXED, NR>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it);
+    const MultiProblem pb(d, mi);
+    const int st = solve_item_fp64<StructuredSource, NT>(pb.src, pb.wi, pb.N, pb.n2, pb.nv, d.beta, pb.o, A,
+                                                         A + (size_t)pb.N * pb.N, sm, piv, perm);
     __syncthreads();  // every thread has read status[item] before it is rewritten
     if (threadIdx.x == 0) {
       status[item] = st;
-      if (iters && !redo_only) iters[item] = it;
+      if (iters && !redo_only) iters[item] = 0;
     }
   }
 }
 
-// Batch whose problems differ in orbital count (the 2-orbital bilayer next to a 1-orbital lattice, say): the same
-// per-item body, with the right-hand-side count chosen per item from its problem's n_orb.  Shared memory and the
-// scratch slot are sized for the largest problem of the launch.
-template <bool MIXED>
-__global__ void __launch_bounds__(BSE_THREADS, MIXED ? DGA_MIXED_MIN_BLOCKS : 3)
-    bse_multi_any_kernel(const dga_bse_problem* __restrict__ probs, const MultiItem* __restrict__ work, int n_items,
-                         int n_max, int max_iter, double tol, int* __restrict__ status, int* __restrict__ iters,
-                         unsigned char* __restrict__ scratch, size_t slot_bytes, int redo_only) {
+template <int NR>
+__device__ __forceinline__ int multi_item_mixed(const dga_bse_problem& d, const MultiItem& mi, int n_max, int max_iter,
+                                                double tol, unsigned char* slot, unsigned char* smem_raw, int* it) {
+  const MultiProblem pb(d, mi);
+  BseSmem<float2>& sm = *reinterpret_cast<BseSmem<float2>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<float2>));
+  int* perm = piv + n_max;
+  double2* colsum = reinterpret_cast<double2*>(smem_raw + mixed_colsum_offset(n_max));
+  float2* A = reinterpret_cast<float2*>(slot);
+  double2* Y = reinterpret_cast<double2*>(slot + (((size_t)pb.N * pb.N * sizeof(float2) + 255) & ~(size_t)255));
+  double2* Rb = Y + (size_t)pb.N * pb.n2;
+  return solve_item_mixed<NR>(pb.src, pb.wi, pb.N, pb.nv, d.beta, max_iter, tol, pb.o, A, Y, Rb, sm, piv, perm, colsum,
+                              it);
+}
+
+// Mixed batch of problems of one orbital count (NR = n_orb^2 > 0), or (NR = 0) of problems that differ in it (the
+// 2-orbital bilayer next to a 1-orbital lattice, say), with the right-hand-side count chosen per item.
+template <int NR>
+__global__ void __launch_bounds__(BSE_THREADS, DGA_MIXED_MIN_BLOCKS)
+    bse_multi_mixed_kernel(const dga_bse_problem* __restrict__ probs, const MultiItem* __restrict__ work, int n_items,
+                           int n_max, int max_iter, double tol, int* __restrict__ status, int* __restrict__ iters,
+                           unsigned char* __restrict__ scratch, size_t slot_bytes) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* slot = scratch + (size_t)blockIdx.x * slot_bytes;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    if (redo_only && (status[item] & DGA_ITEM_REDO) == 0) continue;
     const MultiItem mi = work[item];
     const dga_bse_problem d = probs[mi.prob];
     int it = 0, st = 0;
-    switch (d.n_orb) {
-      case 1: st = multi_item<MIXED, 1>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
-      case 2: st = multi_item<MIXED, 4>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
-      case 3: st = multi_item<MIXED, 9>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
-      default: st = multi_item<MIXED, 16>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
+    if constexpr (NR > 0) {
+      st = multi_item_mixed<NR>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it);
+    } else {
+      switch (d.n_orb) {
+        case 1: st = multi_item_mixed<1>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
+        case 2: st = multi_item_mixed<4>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
+        case 3: st = multi_item_mixed<9>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
+        default: st = multi_item_mixed<16>(d, mi, n_max, max_iter, tol, slot, smem_raw, &it); break;
+      }
     }
-    __syncthreads();  // every thread has read status[item] before it is rewritten
+    __syncthreads();
     if (threadIdx.x == 0) {
       status[item] = st;
-      if (iters && !redo_only) iters[item] = it;
+      if (iters) iters[item] = it;
     }
   }
 }
@@ -820,15 +862,15 @@ __global__ void __launch_bounds__(BSE_THREADS, MIXED ? DGA_MIXED_MIN_BLOCKS : 3)
 //   g3: [2][Q][W][nv][n2][n2]; chi_phys: [2][Q][W][n2][n2]; out: [2][Q][Wpp][Mb][Mb]
 //   slot: A (N x N) | Y (N x NR) | H (2P x n2 x n2) | Z (n2 x n2), complex128
 // ----------------------------------------------------------------------------------------------
-template <int NR>
-__global__ void __launch_bounds__(BSE_THREADS, 3)
+template <int NT>
+__global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     eli_full_vertex_kernel(StructuredSource src, const WorkItem* __restrict__ work, int n_items, int N, int n2, int nv,
-                           int W, int Q, int P, int Wpp, double beta, const double2* __restrict__ g3,
+                           int W, int Q, int P, int Wpp, double beta, int NR, const double2* __restrict__ g3,
                            const double2* __restrict__ chi_phys, double2* __restrict__ out, int* __restrict__ status,
                            double2* __restrict__ scratch, size_t slot_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
-  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
+  Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
   int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
   double2* Y = A + (size_t)N * N;
@@ -863,20 +905,8 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
       }
     }
     __syncthreads();
-    const bool singular = lu_factor<double2>(A, N, N, piv, sm);
-    // row permutation of the factorisation
-    for (int i = tid; i < N; i += T) perm[i] = i;
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 0; i < N; ++i) {
-        const int p = piv[i];
-        if (p != i) {
-          const int t = perm[i];
-          perm[i] = perm[p];
-          perm[p] = t;
-        }
-      }
-    }
+    const bool singular = lu_factor_dmma<NT>(A, N, N, piv, sm.lu);
+    build_perm(N, piv, perm);
     // Z = U_r - U_r chi_r U_r, then H(nu) = Z G3(nu) for the box frequencies
     const double2* uvq = src.uv + ((size_t)wi.ch * Q + wi.q) * n2 * n2;
     const double2* cp = chi_phys + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * n2 * n2;
@@ -911,7 +941,7 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
         Y[(size_t)sidx * N + i] = make_double2((vb < nvp && perm[i] == j) ? 1.0 : 0.0, 0.0);
       }
       __syncthreads();
-      lu_solve_inplace<double2, double2, NR>(A, N, N, Y, sm);
+      lu_solve_n2<NT>(NR, A, N, Y, sm);
       // F columns (s, nu') for the KB box frequencies of this chunk, rows (p, nu) of the box
       for (int e = tid; e < Mb * KB * n2; e += T) {
         const int sidx = e % n2;
@@ -955,9 +985,26 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
 // ----------------------------------------------------------------------------------------------
 constexpr int DENSE_RHS = 16;
 
-__global__ void __launch_bounds__(BSE_THREADS, 3)
+template <int NT>
+__global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     dense_lu_kernel(double2* __restrict__ a, int N, int n_mat, long long mat_stride, int* __restrict__ piv_out,
                     int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
+  for (int m = blockIdx.x; m < n_mat; m += gridDim.x) {
+    const bool singular = lu_factor_dmma<NT>(a + (size_t)m * mat_stride, N, N, piv, sm.lu);
+    __syncthreads();
+    for (int i = threadIdx.x; i < N; i += NT) piv_out[(size_t)m * N + i] = piv[i];
+    if (threadIdx.x == 0) status[m] = singular ? DGA_ITEM_SINGULAR : DGA_ITEM_OK;
+    __syncthreads();
+  }
+}
+
+// The same for N > LU_MAX_N, by the right-looking form.
+__global__ void __launch_bounds__(BSE_THREADS, 3)
+    dense_lu_large_kernel(double2* __restrict__ a, int N, int n_mat, long long mat_stride, int* __restrict__ piv_out,
+                          int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
@@ -980,26 +1027,14 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
                        long long b_sk, int n_rhs, double2* __restrict__ out, long long out_stride,
                        int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
-  int* perm = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
+  Fp64Smem<BSE_THREADS>& sm = *reinterpret_cast<Fp64Smem<BSE_THREADS>*>(smem_raw);
+  int* perm = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<BSE_THREADS>));
   const int tid = threadIdx.x, T = blockDim.x;
   const int n_blk = (n_rhs + DENSE_RHS - 1) / DENSE_RHS;
   for (int t = blockIdx.x; t < n_mat * n_blk; t += gridDim.x) {
     const int m = t / n_blk, k0 = (t - m * n_blk) * DENSE_RHS;
     const int* pv = piv + (size_t)m * N;
-    for (int i = tid; i < N; i += T) perm[i] = i;
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 0; i < N; ++i) {
-        const int p = pv[i];
-        if (p != i) {
-          const int s = perm[i];
-          perm[i] = perm[p];
-          perm[p] = s;
-        }
-      }
-    }
-    __syncthreads();
+    build_perm(N, pv, perm);
     double2* Y = out + (size_t)m * out_stride + (size_t)k0 * N;
     for (int e = tid; e < N * DENSE_RHS; e += T) {
       const int i = e % N, k = e / N, col = k0 + k;
@@ -1014,7 +1049,8 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
       Y[(size_t)k * N + i] = v;
     }
     __syncthreads();
-    lu_solve_inplace<double2, double2, DENSE_RHS>(lu + (size_t)m * lu_stride, N, N, Y, sm);
+    lu_solve_inplace<double2, double2, DENSE_RHS>(lu + (size_t)m * lu_stride, N, N, Y, sm.solve.L11,
+                                                  sm.solve.yb);
     int bad = 0;
     for (int e = tid; e < N * DENSE_RHS; e += T) {
       const double2 v = Y[e];
@@ -1033,10 +1069,10 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
 // the three-leg vertex of the whole pass) is added afterwards by eli_ladder_term_kernel; f1 + term is the sum
 // eli_full_vertex_kernel forms, in the same order, from the same factors.
 // ----------------------------------------------------------------------------------------------
-template <int NRB>
-__device__ void eli_box_epilogue(const StructuredSource& src, const WorkItem& wi, int N, int n2, int nv, int W, int P,
+template <int NT>
+__device__ void eli_box_epilogue(const StructuredSource& src, const WorkItem& wi, int N, int n2, int NRB, int nv, int W, int P,
                                  double beta2, const double2* __restrict__ A, double2* __restrict__ Y,
-                                 const int* __restrict__ perm, double2* __restrict__ o, BseSmem<double2>& sm) {
+                                 const int* __restrict__ perm, double2* __restrict__ o, Fp64Smem<NT>& sm) {
   const int tid = threadIdx.x, T = blockDim.x;
   const int nvp = 2 * P, Mb = n2 * nvp, KB = NRB / n2, off = nv / 2 - P;
   for (int v0 = 0; v0 < nvp; v0 += KB) {
@@ -1048,7 +1084,7 @@ __device__ void eli_box_epilogue(const StructuredSource& src, const WorkItem& wi
       Y[(size_t)sidx * N + i] = make_double2((kk < KB && vb < nvp && perm[i] == j) ? 1.0 : 0.0, 0.0);
     }
     __syncthreads();
-    lu_solve_inplace<double2, double2, NRB>(A, N, N, Y, sm);
+    lu_solve_n2<NT>(NRB, A, N, Y, sm);
     for (int e = tid; e < Mb * KB * n2; e += T) {
       const int sidx = e % n2;
       const int kk = (e / n2) % KB;
@@ -1075,15 +1111,15 @@ __device__ void eli_box_epilogue(const StructuredSource& src, const WorkItem& wi
 
 // FP64 BSE (as bse_solve_sum_fp64_kernel) with the pp-box epilogue for items w < Wpp; NRB = box columns per solve
 // (KB = NRB / n2 box frequencies).  out_pp: [2][Q][Wpp][Mb][Mb].
-template <int NR, int NRB>
-__global__ void __launch_bounds__(BSE_THREADS, 3)
+template <int NT>
+__global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     bse_fp64_eli_kernel(StructuredSource src, const WorkItem* __restrict__ work, int n_items, int N, int n2, int nv,
-                        int W, int Q, double beta, double2* __restrict__ out, int P, int Wpp,
+                        int W, int Q, double beta, double2* __restrict__ out, int NRB, int P, int Wpp,
                         double2* __restrict__ out_pp, int* __restrict__ status, double2* __restrict__ scratch,
                         size_t slot_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BseSmem<double2>& sm = *reinterpret_cast<BseSmem<double2>*>(smem_raw);
-  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(BseSmem<double2>));
+  Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
+  int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
   int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
   double2* Y = A + (size_t)N * N;
@@ -1091,10 +1127,10 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const WorkItem wi = work[item];
     double2* o = out + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * (size_t)N * n2;
-    const int st = solve_item_fp64<StructuredSource, NR>(src, wi, N, nv, beta, o, A, Y, sm, piv, perm);
+    const int st = solve_item_fp64<StructuredSource, NT>(src, wi, N, n2, nv, beta, o, A, Y, sm, piv, perm);
     if (wi.w < Wpp) {
       double2* opp = out_pp + (((size_t)wi.ch * Q + wi.q) * Wpp + wi.w) * (size_t)Mb * Mb;
-      eli_box_epilogue<NRB>(src, wi, N, n2, nv, W, P, beta * beta, A, Y, perm, opp, sm);
+      eli_box_epilogue<NT>(src, wi, N, n2, NRB, nv, W, P, beta * beta, A, Y, perm, opp, sm);
     }
     if (threadIdx.x == 0 && status) status[item] = st;
   }
@@ -1151,48 +1187,55 @@ __global__ void eli_ladder_term_kernel(const double2* __restrict__ uv, const dou
 
 using namespace dga;
 
-static size_t bse_smem_bytes(int N) { return sizeof(BseSmem<double2>) + 2 * sizeof(int) * (size_t)N; }
+// Dynamic shared memory of an FP64 kernel for sizes up to N.
+static size_t bse_smem_bytes(int N) {
+  const int nt = fp64_threads(N);
+  const size_t s = nt == 64 ? sizeof(Fp64Smem<64>) : nt == 128 ? sizeof(Fp64Smem<128>) : sizeof(Fp64Smem<256>);
+  return s + 2 * sizeof(int) * (size_t)N;
+}
+
+// Calls f with the FP64 kernels' thread count for sizes up to N as a compile-time constant.
+template <typename F>
+static auto with_fp64_threads(int N, F f) {
+  switch (fp64_threads(N)) {
+    case 64: return f(std::integral_constant<int, 64>{});
+    case 128: return f(std::integral_constant<int, 128>{});
+    default: return f(std::integral_constant<int, 256>{});
+  }
+}
 
 template <typename K>
-static int grid_for(K kernel, int n_items, size_t smem) {
+static int grid_for(K kernel, int n_items, size_t smem, int threads = BSE_THREADS) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BSE_THREADS, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (per_sm < 1) per_sm = 1;
   int g = sms * per_sm;
   return n_items < g ? n_items : g;
 }
 
-static int bse_grid(int n_items, size_t smem) {
-  return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, 9>, n_items, smem);
+static int bse_grid(int N, int n_items) {
+  return with_fp64_threads(N, [&](auto nt) {
+    return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  });
 }
 
 static bool supported_rhs(int n2) { return n2 == 1 || n2 == 4 || n2 == 9 || n2 == 16; }
 
-// Launches the FP64 kernel instantiated for n2 right-hand sides (1, 4, 9 or 16 orbital pairs).
 template <typename Source>
-static void launch_fp64(int n2, int grid, size_t smem, cudaStream_t stream, const Source& src, const WorkItem* work,
-                        int n_items, int N, int nv, int W, int Q, double beta, double2* out, int* status,
-                        double2* scratch, size_t slot, int redo) {
-#define DGA_FP64_CASE(NRV)                                                                                        \
-  case NRV:                                                                                                       \
-    cudaFuncSetAttribute(bse_solve_sum_fp64_kernel<Source, NRV>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                         (int)smem);                                                                              \
-    bse_solve_sum_fp64_kernel<Source, NRV><<<grid, BSE_THREADS, smem, stream>>>(                                  \
-        src, work, n_items, N, NRV, nv, W, Q, beta, out, status, scratch, slot, redo);                            \
-    break;
-  switch (n2) {
-    DGA_FP64_CASE(1)
-    DGA_FP64_CASE(4)
-    DGA_FP64_CASE(9)
-    DGA_FP64_CASE(16)
-    default:
-      break;
-  }
-#undef DGA_FP64_CASE
+static void launch_fp64(int n2, int grid, cudaStream_t stream, const Source& src, const WorkItem* work, int n_items,
+                        int N, int nv, int W, int Q, double beta, double2* out, int* status, double2* scratch,
+                        size_t slot, int redo) {
+  const size_t smem = bse_smem_bytes(N);
+  with_fp64_threads(N, [&](auto nt) {
+    auto kernel = bse_solve_sum_fp64_kernel<Source, nt.value>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<grid, nt.value, smem, stream>>>(src, work, n_items, N, n2, nv, W, Q, beta, out, status, scratch, slot,
+                                             redo);
+  });
 }
 
 extern "C" {
@@ -1201,8 +1244,7 @@ extern "C" {
 // n2 right-hand sides: one N x N matrix plus N x n2 solution per resident CTA.
 size_t dga_bse_scratch_bytes(int N, int n2, int n_items) {
   if (N <= 0 || n2 <= 0 || n_items <= 0) return 0;
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = bse_grid(n_items, smem);
+  const int grid = bse_grid(N, n_items);
   return (size_t)grid * ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
 }
 
@@ -1220,8 +1262,7 @@ int dga_bse_solve_sum_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, 
     dga_set_error("dga_bse_solve_sum_c128: null pointer argument");
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = bse_grid(n_items, smem);
+  const int grid = bse_grid(N, n_items);
   const size_t slot = (size_t)N * N + (size_t)N * n2;
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_solve_sum_c128: scratch too small (%zu < %zu)", scratch_bytes,
@@ -1237,7 +1278,7 @@ int dga_bse_solve_sum_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, 
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, smem, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -1260,8 +1301,7 @@ int dga_bse_resolve_fp64_c128(int n_orb, int niv, int niw_half, int n_q, int n_c
     dga_set_error("dga_bse_resolve_fp64_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  int grid = bse_grid(n_items, smem);
+  int grid = bse_grid(N, n_items);
   if (grid > grid_limit) grid = grid_limit;
   const size_t slot = (size_t)N * N + (size_t)N * n2;
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
@@ -1277,7 +1317,7 @@ int dga_bse_resolve_fp64_c128(int n_orb, int niv, int niw_half, int n_q, int n_c
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, smem, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 1);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -1298,8 +1338,7 @@ int dga_invert_sum_dense_c128(int n_orb, int niv, int niw_half, int n_q, double 
     dga_set_error("dga_invert_sum_dense_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = bse_grid(n_items, smem);
+  const int grid = bse_grid(N, n_items);
   const size_t slot = (size_t)N * N + (size_t)N * n2;
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_invert_sum_dense_c128: scratch too small");
@@ -1311,7 +1350,7 @@ int dga_invert_sum_dense_c128(int n_orb, int niv, int niw_half, int n_q, double 
   src.nv = nv;
   src.W = niw_half;
   src.Q = n_q;
-  launch_fp64(n2, grid, smem, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -1451,6 +1490,12 @@ int dga_bse_solve_sum_mixed_c128(int n_orb, int niv, int niw_half, int n_q, int 
 // ------------------------------------------------------------------------------------------------
 static int eli_rhs(int n2) { return n2 == 9 ? 9 : 16; }
 
+static int eli_vertex_grid(int N, int n_items) {
+  return with_fp64_threads(N, [&](auto nt) {
+    return grid_for(eli_full_vertex_kernel<nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  });
+}
+
 static size_t eli_slot_elems(int N, int n2, int P) {
   return (size_t)N * N + (size_t)N * eli_rhs(n2) + (size_t)2 * P * n2 * n2 + (size_t)n2 * n2;
 }
@@ -1461,8 +1506,7 @@ extern "C" {
 size_t dga_eli_vertex_scratch_bytes(int n_orb, int niv, int niv_pp, int n_items) {
   const int n2 = n_orb * n_orb, N = n2 * 2 * niv;
   if (!supported_rhs(n2) || n_items <= 0) return 0;
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = grid_for(eli_full_vertex_kernel<16>, n_items, smem);
+  const int grid = eli_vertex_grid(N, n_items);
   return (size_t)grid * eli_slot_elems(N, n2, niv_pp) * sizeof(double2);
 }
 
@@ -1482,8 +1526,7 @@ int dga_eli_full_vertex_c128(int n_orb, int niv, int niw_half, int n_q, int niv_
   }
   const size_t smem = bse_smem_bytes(N);
   const int NR = eli_rhs(n2);
-  int grid = NR == 9 ? grid_for(eli_full_vertex_kernel<9>, n_items, smem)
-                     : grid_for(eli_full_vertex_kernel<16>, n_items, smem);
+  const int grid = eli_vertex_grid(N, n_items);
   const size_t slot = eli_slot_elems(N, n2, niv_pp);
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_eli_full_vertex_c128: scratch too small");
@@ -1498,15 +1541,11 @@ int dga_eli_full_vertex_c128(int n_orb, int niv, int niw_half, int n_q, int niv_
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  if (NR == 9) {
-    eli_full_vertex_kernel<9><<<grid, BSE_THREADS, smem, stream>>>(
-        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, niv_pp, w_pp, beta, (const double2*)g3,
+  with_fp64_threads(N, [&](auto nt) {
+    eli_full_vertex_kernel<nt.value><<<grid, nt.value, smem, stream>>>(
+        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, niv_pp, w_pp, beta, NR, (const double2*)g3,
         (const double2*)chi_phys, (double2*)out, status, (double2*)scratch, slot);
-  } else {
-    eli_full_vertex_kernel<16><<<grid, BSE_THREADS, smem, stream>>>(
-        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, niv_pp, w_pp, beta, (const double2*)g3,
-        (const double2*)chi_phys, (double2*)out, status, (double2*)scratch, slot);
-  }
+  });
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     dga_set_error("dga_eli_full_vertex_c128: launch failed: %s", cudaGetErrorString(err));
@@ -1569,25 +1608,19 @@ static size_t batch_smem(int n_max, int n2, int mixed) {
   return mixed ? mixed_smem_bytes(n_max, n2) : bse_smem_bytes(n_max);
 }
 
-static int batch_grid_hetero(int mixed, int n_items, size_t smem) {
-  return mixed ? grid_for(bse_multi_any_kernel<true>, n_items, smem)
-               : grid_for(bse_multi_any_kernel<false>, n_items, smem);
-}
-
-template <bool MIXED, int NR>
-static int batch_grid(int n_items, size_t smem) {
-  return grid_for(bse_multi_kernel<MIXED, NR>, n_items, smem);
-}
-
-static int batch_grid_any(int mixed, int n2, int n_items, size_t smem) {
-#define DGA_BATCH_GRID(R) \
-  if (n2 == R) return mixed ? batch_grid<true, R>(n_items, smem) : batch_grid<false, R>(n_items, smem);
-  DGA_BATCH_GRID(1)
-  DGA_BATCH_GRID(4)
-  DGA_BATCH_GRID(9)
-  DGA_BATCH_GRID(16)
-#undef DGA_BATCH_GRID
-  return 0;
+// The batch kernels' grids for requests of sizes up to n_max (n2 = 0: of several orbital counts).
+static int batch_grid(int mixed, int n2, int n_max, int n_items, size_t smem) {
+  if (!mixed)
+    return with_fp64_threads(
+        n_max, [&](auto nt) { return grid_for(bse_multi_fp64_kernel<nt.value>, n_items, smem, nt.value); });
+  switch (n2) {
+    case 0: return grid_for(bse_multi_mixed_kernel<0>, n_items, smem);
+    case 1: return grid_for(bse_multi_mixed_kernel<1>, n_items, smem);
+    case 4: return grid_for(bse_multi_mixed_kernel<4>, n_items, smem);
+    case 9: return grid_for(bse_multi_mixed_kernel<9>, n_items, smem);
+    case 16: return grid_for(bse_multi_mixed_kernel<16>, n_items, smem);
+    default: return 0;
+  }
 }
 
 extern "C" {
@@ -1607,8 +1640,8 @@ size_t dga_bse_batch_scratch_bytes(const dga_bse_problem* probs, int n_prob, int
     return (size_t)(kernel == 4 ? dga_block_grid(hetero ? 0 : n2, n_items)
                                 : dga_panel_batch_grid(n2, n_max, n_items, kernel == 3)) *
            slot;
-  if (hetero) return (size_t)batch_grid_hetero(mixed, n_items, batch_smem(n_max, n2_max, mixed)) * slot;
-  return (size_t)batch_grid_any(mixed, n2, n_items, batch_smem(n_max, n2, mixed)) * slot;
+  return (size_t)batch_grid(mixed, hetero ? 0 : n2, n_max, n_items, batch_smem(n_max, hetero ? n2_max : n2, mixed)) *
+         slot;
 }
 
 // One persistent launch over the (problem, ch, q, w) items of several problems of the same orbital count whose
@@ -1644,8 +1677,7 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
   const bool panel = kernel != 2;
   int grid = panel    ? (kernel == 4 ? dga_block_grid(hetero ? 0 : n2, n_items)
                                      : dga_panel_batch_grid(n2, n_max, n_items, kernel == 3))
-             : hetero ? batch_grid_hetero(mixed, n_items, smem)
-                      : batch_grid_any(mixed, n2, n_items, smem);
+                      : batch_grid(mixed, hetero ? 0 : n2, n_max, n_items, smem);
   if (scratch_bytes < slot) {
     dga_set_error("dga_bse_solve_sum_batch_c128: scratch too small (%zu < one slot of %zu)", scratch_bytes, slot);
     return DGA_ERR_SCRATCH;
@@ -1667,36 +1699,23 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
     }
     return DGA_OK;
   }
-  if (hetero) {
-    if (mixed)
-      bse_multi_any_kernel<true><<<grid, BSE_THREADS, smem, stream>>>(pd, wk, n_items, n_max, max_iter, tol, status,
-                                                                      iters, sc, slot, 0);
-    else
-      bse_multi_any_kernel<false><<<grid, BSE_THREADS, smem, stream>>>(pd, wk, n_items, n_max, max_iter, tol, status,
-                                                                       iters, sc, slot, redo);
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) {
-      dga_set_error("dga_bse_solve_sum_batch_c128: launch failed: %s", cudaGetErrorString(err));
-      return DGA_ERR_LAUNCH;
+  if (mixed) {
+    const auto go = [&](auto kernel) {
+      kernel<<<grid, BSE_THREADS, smem, stream>>>(pd, wk, n_items, n_max, max_iter, tol, status, iters, sc, slot);
+    };
+    switch (hetero ? 0 : n2) {
+      case 0: go(bse_multi_mixed_kernel<0>); break;
+      case 1: go(bse_multi_mixed_kernel<1>); break;
+      case 4: go(bse_multi_mixed_kernel<4>); break;
+      case 9: go(bse_multi_mixed_kernel<9>); break;
+      case 16: go(bse_multi_mixed_kernel<16>); break;
     }
-    return DGA_OK;
+  } else {
+    with_fp64_threads(n_max, [&](auto nt) {
+      bse_multi_fp64_kernel<nt.value><<<grid, nt.value, smem, stream>>>(pd, wk, n_items, n_max, status, iters, sc, slot,
+                                                                        redo);
+    });
   }
-#define DGA_BATCH_CASE(R)                                                                                          \
-  case R:                                                                                                          \
-    if (mixed)                                                                                                     \
-      bse_multi_kernel<true, R><<<grid, BSE_THREADS, smem, stream>>>(pd, wk, n_items, n_max, max_iter, tol, status, \
-                                                                     iters, sc, slot, 0);                         \
-    else                                                                                                           \
-      bse_multi_kernel<false, R><<<grid, BSE_THREADS, smem, stream>>>(pd, wk, n_items, n_max, max_iter, tol,       \
-                                                                      status, iters, sc, slot, redo);             \
-    break;
-  switch (n2) {
-    DGA_BATCH_CASE(1)
-    DGA_BATCH_CASE(4)
-    DGA_BATCH_CASE(9)
-    DGA_BATCH_CASE(16)
-  }
-#undef DGA_BATCH_CASE
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     dga_set_error("dga_bse_solve_sum_batch_c128: launch failed: %s", cudaGetErrorString(err));
@@ -1760,7 +1779,7 @@ static int tuned_grid(int kernel, int mixed, int N, int n2, int n_items, const d
   } else {
     *smem = bse_smem_bytes(N);
     *slot = ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
-    grid = bse_grid(n_items, *smem);
+    grid = bse_grid(N, n_items);
   }
   const int cps = t ? t->ctas_per_sm : 0;
   if (cps > 0) {
@@ -1840,7 +1859,7 @@ int dga_bse_solve_sum_tuned_c128(int n_orb, int niv, int niw_half, int n_q, int 
 #undef DGA_TUNED_MIXED_CASE
     err = cudaGetLastError();
   } else {
-    launch_fp64(n2, grid, smem, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+    launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
                 (double2*)out, status, (double2*)scratch, slot / sizeof(double2), 0);
     err = cudaGetLastError();
   }
@@ -1929,8 +1948,7 @@ int dga_bse_solve_sum_noalloc_c128(int n_orb, int niv, int niw_half, int n_q, in
   void* scratch = nullptr;
   int rc = noalloc_scratch_ptr(&scratch);
   if (rc != DGA_OK) return rc;
-  const size_t smem = bse_smem_bytes(N);
-  int grid = bse_grid(n_items, smem);
+  int grid = bse_grid(N, n_items);
   if ((size_t)grid > capacity_slots) grid = (int)capacity_slots;
   StructuredSource src;
   src.gamma_cm = (const double2*)gamma_cm;
@@ -1941,7 +1959,7 @@ int dga_bse_solve_sum_noalloc_c128(int n_orb, int niv, int niw_half, int n_q, in
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, smem, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -1961,9 +1979,17 @@ int dga_lu_batched_c128(void* a, int N, int n_mat, long long mat_stride, int* pi
     dga_set_error("dga_lu_batched_c128: invalid arguments (N=%d n_mat=%d)", N, n_mat);
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = grid_for(dense_lu_kernel, n_mat, smem);
-  dense_lu_kernel<<<grid, BSE_THREADS, smem, stream>>>((double2*)a, N, n_mat, mat_stride, piv, status);
+  if (N <= LU_MAX_N) {
+    const size_t smem = bse_smem_bytes(N);
+    with_fp64_threads(N, [&](auto nt) {
+      const int grid = grid_for(dense_lu_kernel<nt.value>, n_mat, smem, nt.value);
+      dense_lu_kernel<nt.value><<<grid, nt.value, smem, stream>>>((double2*)a, N, n_mat, mat_stride, piv, status);
+    });
+  } else {
+    const size_t smem = sizeof(BseSmem<double2>) + sizeof(int) * (size_t)N;
+    const int grid = grid_for(dense_lu_large_kernel, n_mat, smem);
+    dense_lu_large_kernel<<<grid, BSE_THREADS, smem, stream>>>((double2*)a, N, n_mat, mat_stride, piv, status);
+  }
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     dga_set_error("dga_lu_batched_c128: launch failed: %s", cudaGetErrorString(err));
@@ -1982,7 +2008,7 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
     dga_set_error("dga_lu_solve_batched_c128: invalid arguments (N=%d n_mat=%d n_rhs=%d)", N, n_mat, n_rhs);
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
+  const size_t smem = sizeof(Fp64Smem<BSE_THREADS>) + sizeof(int) * (size_t)N;
   const long long n_tasks = (long long)n_mat * (cols / DENSE_RHS);
   if (n_tasks > 0x7fffffffLL) {
     dga_set_error("dga_lu_solve_batched_c128: too many right-hand-side blocks");
@@ -2002,13 +2028,18 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
 
 }  // extern "C"
 
+static int eli_grid(int N, int n_items) {
+  return with_fp64_threads(N, [&](auto nt) {
+    return grid_for(bse_fp64_eli_kernel<nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  });
+}
+
 extern "C" {
 
 // Scratch bytes of dga_bse_solve_sum_eli_c128 for n_items items of size N.
 size_t dga_bse_eli_scratch_bytes(int N, int n2, int n_items) {
   if (N <= 0 || !supported_rhs(n2) || n_items <= 0) return 0;
-  const size_t smem = bse_smem_bytes(N);
-  const int grid = grid_for(bse_fp64_eli_kernel<9, 9>, n_items, smem);
+  const int grid = eli_grid(N, n_items);
   return (size_t)grid * ((size_t)N * N + (size_t)N * eli_rhs(n2)) * sizeof(double2);
 }
 
@@ -2028,13 +2059,7 @@ int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_
   }
   const size_t smem = bse_smem_bytes(N);
   const size_t slot = (size_t)N * N + (size_t)N * eli_rhs(n2);
-  int grid = 0;
-  switch (n2) {
-    case 1: grid = grid_for(bse_fp64_eli_kernel<1, 16>, n_items, smem); break;
-    case 4: grid = grid_for(bse_fp64_eli_kernel<4, 16>, n_items, smem); break;
-    case 9: grid = grid_for(bse_fp64_eli_kernel<9, 9>, n_items, smem); break;
-    default: grid = grid_for(bse_fp64_eli_kernel<16, 16>, n_items, smem); break;
-  }
+  const int grid = eli_grid(N, n_items);
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_solve_sum_eli_c128: scratch too small");
     return DGA_ERR_SCRATCH;
@@ -2048,19 +2073,11 @@ int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-#define DGA_ELI_CASE(NRV, NRB)                                                                                 \
-  case NRV:                                                                                                    \
-    bse_fp64_eli_kernel<NRV, NRB><<<grid, BSE_THREADS, smem, stream>>>(                                        \
-        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, beta, (double2*)out, niv_pp, w_pp,      \
-        (double2*)out_pp, status, (double2*)scratch, slot);                                                    \
-    break;
-  switch (n2) {
-    DGA_ELI_CASE(1, 16)
-    DGA_ELI_CASE(4, 16)
-    DGA_ELI_CASE(9, 9)
-    DGA_ELI_CASE(16, 16)
-  }
-#undef DGA_ELI_CASE
+  with_fp64_threads(N, [&](auto nt) {
+    bse_fp64_eli_kernel<nt.value><<<grid, nt.value, smem, stream>>>(
+        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, beta, (double2*)out, eli_rhs(n2), niv_pp, w_pp,
+        (double2*)out_pp, status, (double2*)scratch, slot);
+  });
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     dga_set_error("dga_bse_solve_sum_eli_c128: launch failed: %s", cudaGetErrorString(err));
