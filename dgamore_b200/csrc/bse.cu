@@ -336,14 +336,15 @@ __device__ bool lu_factor(C* __restrict__ A, int N, int ld, int* __restrict__ pi
 }
 
 // ----------------------------------------------------------------------------------------------
-// Solve (L U) Y = B in place for the n_rhs columns of Y (column-major, leading dimension N), with the LU
-// factors of lu_factor (unit lower L below the diagonal, U on and above).  Blocked by 32 rows: the diagonal
+// Solves for the n_rhs columns of Y in place (column-major, leading dimension N), with the LU factors of lu_factor or
+// lu_factor_dmma (unit lower L below the diagonal, U on and above): lu_forward_inplace Y = L^-1 Y, lu_backward_inplace
+// Y = U^-1 Y.  Blocked by 32 rows: the diagonal
 // block is solved by one warp per right-hand side (lane = row, the solved value broadcast by shuffle), the
 // rest of the rows are updated from the block copy in shared memory.  L11: the diagonal block, yb: [n_rhs][32] the
 // solved block, both in shared memory.
 // ----------------------------------------------------------------------------------------------
 template <typename C, typename CY, int NR>
-__device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y,
+__device__ void lu_forward_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y,
                                  C (*__restrict__ L11)[BSE_NB + 1], CY* __restrict__ yb) {
   constexpr int n_rhs = NR;
   // factor elements a thread has in flight in the row updates: eight where each one feeds several right-hand
@@ -411,7 +412,19 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
     }
     __syncthreads();
   }
-  // backward: U y = z
+}
+
+template <typename C, typename CY, int NR>
+__device__ void lu_backward_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y,
+                                 C (*__restrict__ L11)[BSE_NB + 1], CY* __restrict__ yb) {
+  constexpr int n_rhs = NR;
+  // factor elements a thread has in flight in the row updates: eight where each one feeds several right-hand
+  // sides; with one to three the registers go to the factorisation around the solve instead
+  constexpr int SOLVE_LOADS = NR >= 4 ? 8 : 1;
+  using R = decltype(C::x);
+  using RY = decltype(CY::x);
+  const int tid = threadIdx.x, T = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
   const int nblk = (N + BSE_NB - 1) / BSE_NB;
   for (int blk = nblk - 1; blk >= 0; --blk) {
     const int b0 = blk * BSE_NB;
@@ -423,11 +436,10 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
     __syncthreads();
     for (int s = warp; s < n_rhs; s += nwarps) {
       CY y = lane < bn ? Y[(size_t)s * N + b0 + lane] : cmake<CY>(RY(0), RY(0));
+      const C d = lane < bn ? L11[lane][lane] : cmake<C>(R(1), R(0));
+      const double2 rd = crecip(make_double2((double)d.x, (double)d.y));  // every row's at once, not one after the other
       for (int r = bn - 1; r >= 0; --r) {
-        if (lane == r) {
-          const C u = L11[r][r];
-          y = cdiv(y, cmake<CY>((RY)u.x, (RY)u.y));
-        }
+        if (lane == r) y = cmul_fma(y, rd);
         CY yr;
         yr.x = __shfl_sync(0xffffffffu, y.x, r);
         yr.y = __shfl_sync(0xffffffffu, y.y, r);
@@ -477,6 +489,13 @@ __device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __r
   }
 }
 
+template <typename C, typename CY, int NR>
+__device__ void lu_solve_inplace(const C* __restrict__ A, int N, int ld, CY* __restrict__ Y,
+                                 C (*__restrict__ L11)[BSE_NB + 1], CY* __restrict__ yb) {
+  lu_forward_inplace<C, CY, NR>(A, N, ld, Y, L11, yb);
+  lu_backward_inplace<C, CY, NR>(A, N, ld, Y, L11, yb);
+}
+
 // perm[i] = the original row at position i after the interchanges in piv (both N ints in shared memory).  One warp looks
 // for the rows that moved, 32 at a time, and swaps those in order.
 __device__ void build_perm(int N, const int* __restrict__ piv, int* __restrict__ perm) {
@@ -516,74 +535,171 @@ __device__ void permuted_selector(CY* __restrict__ Y, int N, int nv, int n_rhs, 
   __syncthreads();
 }
 
+// Threads of an FP64 CTA: one warp up to N = 64 (29,600 factorisations of N = 40: 1.71 ms, 1.89 with two warps), two up to
+// N = 192 (14,208 of N = 120: 7.6 ms, 8.2 with one and 7.9 with four), four up to N = 512 (1,184 of N = 480: 18.2 ms, 18.6
+// with eight), eight above (592 of N = 720: 27.7 ms, 27.3 with four, whose panels hold eight rows a thread). Where the
+// items would fill less than half of the SMs' threads that way, each gets more: up to two rows a thread (441 items of
+// N = 200: 1.8 ms with four warps, 2.5 with two).
+static int fp64_threads(int N, int n_items) {
+  int nt = N <= 64 ? 32 : N <= LU_SMALL_N ? 64 : N <= 512 ? 128 : 256;
+  while (nt < 256 && nt < N && (long)n_items * nt <= (long)device_sm_count() * 256) nt *= 2;
+  return nt;
+}
+constexpr int fp64_min_blocks(int NT) { return 512 / NT; }  // 128 registers a thread
+
 // Shared memory of the FP64 kernels: the factorisation's and the solves' buffers are never live at the same time.  The
-// pivots and the permutation (N ints each) follow it.
+// pivots (N ints) follow it.
 template <int NT>
 struct Fp64Smem {
   union {
-    LuSmem<NT> lu;
+    LuSmem<NT, 16> lu16;
+    LuSmem<NT, NT <= 64 ? 16 : 32> lu32;  // CTAs of one or two warps take no matrix beyond LU_SMALL_N
     struct {
-      double2 L11[BSE_NB][BSE_NB + 1];
       double2 yb[MAX_RHS * BSE_NB];
+      double2 L11[NT <= 64 ? 1 : BSE_NB][BSE_NB + 1];
     } solve;
   };
   int flag;
 };
 
-// Threads of an FP64 CTA.  Each thread holds one row of a panel up to N = 64 and 128; from there a CTA of 128 threads is
-// the faster one up to about N = 350 (four CTAs an SM hide one another's panels: 9.7 against 11.3 ms for 3,552 factorisations
-// of N = 240), a CTA of 256 above (18.2 against 20.6 ms for 1,184 of N = 480; 27.0 against 39.5 ms for 592 of N = 720), and
-// 64 threads up to N = 64 (2.95 against 3.28 ms for 29,600 of N = 40).
-constexpr int fp64_threads(int N) { return N <= 64 ? 64 : N <= 352 ? 128 : 256; }
-constexpr int fp64_min_blocks(int NT) { return 512 / NT; }  // 128 registers a thread
-
-// ----------------------------------------------------------------------------------------------
-// One work item in FP64: form A, LU, selector solve, X = Y / beta into out (rows (p,nu), n2 columns).
-// Returns the item's status bits.  All threads of the CTA call it.
-// ----------------------------------------------------------------------------------------------
-// The right-hand-side count is chosen per item (n2 = 1, 4, 9 or 16), which keeps one copy of the factorisation per kernel.
+// LU and backward substitution with the block width of N.
 template <int NT>
-__device__ void lu_solve_n2(int n2, const double2* __restrict__ A, int N, double2* __restrict__ Y, Fp64Smem<NT>& sm) {
-  switch (n2) {
-    case 1: lu_solve_inplace<double2, double2, 1>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
-    case 4: lu_solve_inplace<double2, double2, 4>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
-    case 9: lu_solve_inplace<double2, double2, 9>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
-    default: lu_solve_inplace<double2, double2, 16>(A, N, N, Y, sm.solve.L11, sm.solve.yb); break;
+__device__ __forceinline__ bool fp64_lu(double2* __restrict__ A, int N, int ncols, int* __restrict__ piv,
+                                        Fp64Smem<NT>& sm) {
+  if (NT <= 64 || N <= LU_SMALL_N) return lu_factor_dmma<NT, 16>(A, N, ncols, N, piv, sm.lu16);
+  return lu_factor_dmma<NT, NT <= 64 ? 16 : 32>(A, N, ncols, N, piv, sm.lu32);
+}
+template <int NT>
+__device__ __forceinline__ void fp64_backward(const double2* __restrict__ A, int N, double2* Y, int ncols,
+                                              Fp64Smem<NT>& sm) {
+  if (NT <= 64 || N <= LU_SMALL_N)
+    lu_backward_dmma<NT, 16>(A, N, N, Y, N, ncols, sm.lu16);
+  else
+    lu_backward_dmma<NT, NT <= 64 ? 16 : 32>(A, N, N, Y, N, ncols, sm.lu32);
+}
+
+// Y = U^-1 Y for a few right-hand sides in a CTA of one or two warps: as lu_backward_inplace, but the diagonal block's
+// columns come straight from L2, eight steps ahead of the chain, so that no shared memory limits the CTAs of an SM. (With
+// eight warps the staged form is the faster one: 711 against 750 ms for the three-orbital pass's items, whose blocks come
+// from HBM.)
+template <int NR>
+__device__ void lu_backward_direct(const double2* __restrict__ A, int N, double2* __restrict__ Y,
+                                   double2* __restrict__ yb) {
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = T >> 5;
+  for (int b0 = (N - 1) / 32 * 32; b0 >= 0; b0 -= 32) {
+    const int bn = min(32, N - b0);
+    for (int s = warp; s < NR; s += nwarps) {
+      const double2* D = A + (size_t)b0 * N + b0 + min(lane, bn - 1);
+      double2 y = lane < bn ? Y[(size_t)s * N + b0 + lane] : make_double2(0.0, 0.0);
+      const double2 rd = crecip(D[(size_t)min(lane, bn - 1) * N]);  // every row's at once, not one after the other
+      double2 u[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) u[k] = D[(size_t)min(24 + k, bn - 1) * N];
+#pragma unroll 1
+      for (int r0 = 24; r0 >= 0; r0 -= 8) {
+        double2 n[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) n[k] = D[(size_t)min(max(r0 - 8, 0) + k, bn - 1) * N];
+#pragma unroll
+        for (int k = 7; k >= 0; --k) {
+          const int r = r0 + k;
+          if (r >= bn) continue;
+          if (lane == r) y = cmul_fma(y, rd);
+          double2 yr;
+          yr.x = __shfl_sync(0xffffffffu, y.x, r);
+          yr.y = __shfl_sync(0xffffffffu, y.y, r);
+          if (lane < r) cfms(y, u[k], yr);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) u[k] = n[k];
+      }
+      if (lane < bn) {
+        Y[(size_t)s * N + b0 + lane] = y;
+        yb[s * 32 + lane] = y;
+      }
+    }
+    __syncthreads();
+    // rows above the block: one thread per row, every right-hand side at once, eight factor elements in flight
+    for (int i = tid; i < b0; i += T) {
+      double2 acc[NR];
+#pragma unroll
+      for (int s = 0; s < NR; ++s) acc[s] = Y[(size_t)s * N + i];
+      for (int r0 = 0; r0 < bn; r0 += 8) {
+        double2 u[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) u[k] = A[(size_t)(b0 + min(r0 + k, bn - 1)) * N + i];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (r0 + k >= bn) break;
+#pragma unroll
+          for (int s = 0; s < NR; ++s) cfms(acc[s], u[k], yb[s * 32 + r0 + k]);
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < NR; ++s) Y[(size_t)s * N + i] = acc[s];
+    }
+    __syncthreads();
   }
 }
 
-template <typename Source, int NT>
-__device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int n2, int nv, double beta,
-                               double2* __restrict__ o, double2* __restrict__ A, double2* __restrict__ Y,
-                               Fp64Smem<NT>& sm, int* piv, int* perm) {
+// The right-hand-side count is chosen per item (n2 = 1, 4, 9 or 16), which keeps one copy of the factorisation per kernel.
+template <int NR, int NT>
+__device__ __forceinline__ void lu_backward_rhs(const double2* __restrict__ A, int N, double2* __restrict__ Y,
+                                                Fp64Smem<NT>& sm) {
+  if constexpr (NT <= 64)
+    lu_backward_direct<NR>(A, N, Y, sm.solve.yb);
+  else
+    lu_backward_inplace<double2, double2, NR>(A, N, N, Y, sm.solve.L11, sm.solve.yb);
+}
+template <int NT>
+__device__ __forceinline__ void lu_backward_n2(int n2, const double2* __restrict__ A, int N, double2* __restrict__ Y,
+                                               Fp64Smem<NT>& sm) {
+  switch (n2) {
+    case 1: lu_backward_rhs<1, NT>(A, N, Y, sm); break;
+    case 4: lu_backward_rhs<4, NT>(A, N, Y, sm); break;
+    case 9: lu_backward_rhs<9, NT>(A, N, Y, sm); break;
+    default: lu_backward_rhs<16, NT>(A, N, Y, sm); break;
+  }
+}
+
+// A work item's matrix, column-major with leading dimension N, formed eight columns at a time (eight loads of Gamma_r in
+// flight per thread; one column at a time the loop waited for L2 once per column), and the n2 selector right-hand sides
+// (S[j, s] = 1 if the orbital pair of row j is s) in the columns behind it.
+template <typename Source>
+__device__ void form_item_fp64(const Source& src, const WorkItem& wi, int N, int n2, int nv, double2* __restrict__ A) {
   const int tid = threadIdx.x, T = blockDim.x;
-  // form A column by column; the (pair, nu) split of a thread's rows advances by T = q_T nv + r_T per step
-  {
-    const int pr0 = tid / nv, vr0 = tid - pr0 * nv;
-    const int qT = T / nv, rT = T - qT * nv;
+  for (int i = tid; i < N; i += T) {
+    const int pr = i / nv, vr = i - pr * nv;
     int pc = 0, vc = 0;
-    for (int j = 0; j < N; ++j) {
-      double2* col = A + (size_t)j * N;
-      int pr = pr0, vr = vr0;
-      for (int i = tid; i < N; i += T) {
-        col[i] = src.element(wi.ch, wi.q, wi.w, N, i, j, pr, vr, pc, vc);
-        pr += qT;
-        vr += rT;
-        if (vr >= nv) {
-          vr -= nv;
-          ++pr;
+    for (int j0 = 0; j0 < N; j0 += 8) {
+      double2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (j0 + u < N) v[u] = src.element(wi.ch, wi.q, wi.w, N, i, j0 + u, pr, vr, pc, vc);
+        if (++vc == nv) {
+          vc = 0;
+          ++pc;
         }
       }
-      if (++vc == nv) {
-        vc = 0;
-        ++pc;
-      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (j0 + u < N) A[(size_t)(j0 + u) * N + i] = v[u];
     }
+    for (int s = 0; s < n2; ++s) A[(size_t)(N + s) * N + i] = make_double2(pr == s ? 1.0 : 0.0, 0.0);
   }
+}
+
+// n_box further right-hand sides behind the selectors leave as L^-1 P B (the caller's backward substitution is left).
+template <typename Source, int NT>
+__device__ int solve_item_fp64(const Source& src, const WorkItem& wi, int N, int n2, int nv, double beta,
+                               double2* __restrict__ o, double2* __restrict__ A, Fp64Smem<NT>& sm, int* piv,
+                               int n_box = 0) {
+  const int tid = threadIdx.x, T = blockDim.x;
+  double2* Y = A + (size_t)N * N;
+  form_item_fp64(src, wi, N, n2, nv, A);
   __syncthreads();
-  const bool singular = lu_factor_dmma<NT>(A, N, N, piv, sm.lu);
-  permuted_selector<double2>(Y, N, nv, n2, piv, perm);
-  lu_solve_n2<NT>(n2, A, N, Y, sm);
+  const bool singular = fp64_lu<NT>(A, N, N + n2 + n_box, piv, sm);
+  lu_backward_n2<NT>(n2, A, N, Y, sm);
   // X[i][s] = Y[i][s] / beta, finiteness check
   if (tid == 0) sm.flag = 0;
   __syncthreads();
@@ -613,15 +729,13 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
-  int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
-  double2* Y = A + (size_t)N * N;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     // re-solve mode: only the items whose status says the mixed solve did not converge or was not finite
     if (redo_only && (status[item] & DGA_ITEM_REDO) == 0) continue;
     const WorkItem wi = work[item];
     double2* o = out + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * (size_t)N * n2;
-    const int st = solve_item_fp64<Source, NT>(src, wi, N, n2, nv, beta, o, A, Y, sm, piv, perm);
+    const int st = solve_item_fp64<Source, NT>(src, wi, N, n2, nv, beta, o, A, sm, piv);
     if (threadIdx.x == 0 && status) status[item] = st;
   }
 }
@@ -790,15 +904,13 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
-  int* perm = piv + n_max;
   double2* A = reinterpret_cast<double2*>(scratch + (size_t)blockIdx.x * slot_bytes);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     if (redo_only && (status[item] & DGA_ITEM_REDO) == 0) continue;
     const MultiItem mi = work[item];
     const dga_bse_problem d = probs[mi.prob];
     const MultiProblem pb(d, mi);
-    const int st = solve_item_fp64<StructuredSource, NT>(pb.src, pb.wi, pb.N, pb.n2, pb.nv, d.beta, pb.o, A,
-                                                         A + (size_t)pb.N * pb.N, sm, piv, perm);
+    const int st = solve_item_fp64<StructuredSource, NT>(pb.src, pb.wi, pb.N, pb.n2, pb.nv, d.beta, pb.o, A, sm, piv);
     __syncthreads();  // every thread has read status[item] before it is rewritten
     if (threadIdx.x == 0) {
       status[item] = st;
@@ -857,56 +969,64 @@ __global__ void __launch_bounds__(BSE_THREADS, DGA_MIXED_MIN_BLOCKS)
 // Eliashberg full vertex in the pp frequency box (one CTA per (channel, q, w) item):
 //   F[(p,nu),(s,nu')] = beta^2 (delta_{nu nu'} c0(nu)[p][s] - sum_{m,m'} c0(nu)[p][m] chi*[(m,nu),(m',nu')] c0(nu')[m'][s])
 //                       + (Z G3(nu) G3(nu'))[p][s],   Z = U_r - U_r chi_r U_r,  c0 = chi0^-1,  G3 = gamma_r
-// for nu, nu' in the box [niv - P, niv + P) (eliashberg_solver.py:175-204).  chi* = A^-1 is never formed: the
-// LU factors of A are solved against the unit vectors of KB box frequencies at a time (NR = KB n2 columns).
+// for nu, nu' in the box [niv - P, niv + P) (eliashberg_solver.py:175-204).  chi* = A^-1 is never formed: the unit vectors
+// of the box frequencies are right-hand sides of the LU (their forward substitution runs with the factorisation's block
+// rows, all columns at once on the FP64 tensor pipe).
 //   g3: [2][Q][W][nv][n2][n2]; chi_phys: [2][Q][W][n2][n2]; out: [2][Q][Wpp][Mb][Mb]
-//   slot: A (N x N) | Y (N x NR) | H (2P x n2 x n2) | Z (n2 x n2), complex128
+//   slot: A (N x N) | Y (N x Mb) | H (2P x n2 x n2) | Z (n2 x n2), complex128
 // ----------------------------------------------------------------------------------------------
+// The unit vectors of the box columns: column vb n2 + m' of Y has its one at row (m', off + vb).
+__device__ void eli_box_columns(int N, int n2, int nv, int P, double2* __restrict__ Y) {
+  const int off = nv / 2 - P, Mb = n2 * 2 * P;
+  for (int e = threadIdx.x; e < N * Mb; e += blockDim.x) {
+    const int i = e % N, col = e / N, vb = col / n2, mp = col - vb * n2;
+    Y[e] = make_double2(i == mp * nv + off + vb ? 1.0 : 0.0, 0.0);
+  }
+}
+
+// beta^2 (delta_{nu nu'} c0(nu)[p][s] - sum_{m,m'} c0(nu)[p][m] chi*[(m,nu),(m',nu')] c0(nu')[m'][s]) with chi* in the box
+// columns Y.
+__device__ __forceinline__ double2 eli_box_element(const StructuredSource& src, const WorkItem& wi, int W, int n2, int nv,
+                                                   int N, int off, int P, double beta2, const double2* Y, int p, int vb,
+                                                   int sidx, int vbp) {
+  const int vr = off + vb, vc = off + vbp;
+  const double2* c0r = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vr) * n2 * n2;
+  const double2* c0c = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vc) * n2 * n2;
+  double2 t = make_double2(0.0, 0.0);
+  for (int m = 0; m < n2; ++m) {
+    double2 inner = make_double2(0.0, 0.0);
+    for (int mp = 0; mp < n2; ++mp) cfma(inner, Y[(size_t)(vbp * n2 + mp) * N + m * nv + vr], c0c[mp * n2 + sidx]);
+    cfma(t, c0r[p * n2 + m], inner);
+  }
+  double2 f1 = make_double2(-t.x, -t.y);
+  if (vb == vbp) f1 = cadd(f1, c0r[p * n2 + sidx]);
+  return cscale(f1, beta2);
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     eli_full_vertex_kernel(StructuredSource src, const WorkItem* __restrict__ work, int n_items, int N, int n2, int nv,
-                           int W, int Q, int P, int Wpp, double beta, int NR, const double2* __restrict__ g3,
+                           int W, int Q, int P, int Wpp, double beta, const double2* __restrict__ g3,
                            const double2* __restrict__ chi_phys, double2* __restrict__ out, int* __restrict__ status,
                            double2* __restrict__ scratch, size_t slot_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
-  int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
   double2* Y = A + (size_t)N * N;
-  const int nvp = 2 * P, Mb = n2 * nvp, KB = NR / n2, off = nv / 2 - P;
-  double2* H = Y + (size_t)N * NR;
+  const int nvp = 2 * P, Mb = n2 * nvp, off = nv / 2 - P;
+  double2* H = Y + (size_t)N * Mb;
   double2* Z = H + (size_t)nvp * n2 * n2;
   const int tid = threadIdx.x, T = blockDim.x;
   const double beta2 = beta * beta;
 
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const WorkItem wi = work[item];
-    {
-      const int pr0 = tid / nv, vr0 = tid - pr0 * nv;
-      const int qT = T / nv, rT = T - qT * nv;
-      int pc = 0, vc = 0;
-      for (int j = 0; j < N; ++j) {
-        double2* col = A + (size_t)j * N;
-        int pr = pr0, vr = vr0;
-        for (int i = tid; i < N; i += T) {
-          col[i] = src.element(wi.ch, wi.q, wi.w, N, i, j, pr, vr, pc, vc);
-          pr += qT;
-          vr += rT;
-          if (vr >= nv) {
-            vr -= nv;
-            ++pr;
-          }
-        }
-        if (++vc == nv) {
-          vc = 0;
-          ++pc;
-        }
-      }
-    }
+    form_item_fp64(src, wi, N, 0, nv, A);
+    eli_box_columns(N, n2, nv, P, Y);
     __syncthreads();
-    const bool singular = lu_factor_dmma<NT>(A, N, N, piv, sm.lu);
-    build_perm(N, piv, perm);
+    const bool singular = fp64_lu<NT>(A, N, N + Mb, piv, sm);
+    fp64_backward<NT>(A, N, Y, Mb, sm);
     // Z = U_r - U_r chi_r U_r, then H(nu) = Z G3(nu) for the box frequencies
     const double2* uvq = src.uv + ((size_t)wi.ch * Q + wi.q) * n2 * n2;
     const double2* cp = chi_phys + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * n2 * n2;
@@ -931,47 +1051,18 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     }
     __syncthreads();
     double2* o = out + (((size_t)wi.ch * Q + wi.q) * Wpp + wi.w) * (size_t)Mb * Mb;
-    for (int v0 = 0; v0 < nvp; v0 += KB) {
-      // unit vectors of the box columns (m', nu') for nu' in [v0, v0 + KB), permuted by the pivots
-      for (int e = tid; e < N * NR; e += T) {
-        const int i = e % N, sidx = e / N;
-        const int kk = sidx / n2, mp = sidx - kk * n2;
-        const int vb = v0 + kk;
-        const int j = mp * nv + off + vb;
-        Y[(size_t)sidx * N + i] = make_double2((vb < nvp && perm[i] == j) ? 1.0 : 0.0, 0.0);
-      }
-      __syncthreads();
-      lu_solve_n2<NT>(NR, A, N, Y, sm);
-      // F columns (s, nu') for the KB box frequencies of this chunk, rows (p, nu) of the box
-      for (int e = tid; e < Mb * KB * n2; e += T) {
-        const int sidx = e % n2;
-        const int kk = (e / n2) % KB;
-        const int row = e / (n2 * KB);
-        const int vbp = v0 + kk;
-        if (vbp >= nvp) continue;
-        const int p = row / nvp, vb = row - p * nvp;
-        const int vr = off + vb, vc = off + vbp;
-        const double2* c0r = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vr) * n2 * n2;
-        const double2* c0c = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vc) * n2 * n2;
-        // t = sum_{m,m'} c0r[p][m] chi*[(m,vr),(m',vc)] c0c[m'][s]
-        double2 t = make_double2(0.0, 0.0);
-        for (int m = 0; m < n2; ++m) {
-          double2 inner = make_double2(0.0, 0.0);
-          for (int mp = 0; mp < n2; ++mp) cfma(inner, Y[(size_t)(kk * n2 + mp) * N + m * nv + vr], c0c[mp * n2 + sidx]);
-          cfma(t, c0r[p * n2 + m], inner);
-        }
-        double2 f1 = make_double2(-t.x, -t.y);
-        if (vb == vbp) f1 = cadd(f1, c0r[p * n2 + sidx]);
-        f1 = cscale(f1, beta2);
-        // (Z G3(nu)) G3(nu')
-        const double2* hrow = H + (size_t)vb * n2 * n2 + p * n2;
-        const double2* gcol = g3q + (size_t)vc * n2 * n2;
-        double2 f2 = make_double2(0.0, 0.0);
-        for (int u = 0; u < n2; ++u) cfma(f2, hrow[u], gcol[u * n2 + sidx]);
-        o[(size_t)row * Mb + sidx * nvp + vbp] = cadd(f1, f2);
-      }
-      __syncthreads();
+    for (int e = tid; e < Mb * Mb; e += T) {
+      const int sidx = e % n2, vbp = (e / n2) % nvp, row = e / Mb;
+      const int p = row / nvp, vb = row - p * nvp, vc = off + vbp;
+      const double2 f1 = eli_box_element(src, wi, W, n2, nv, N, off, P, beta2, Y, p, vb, sidx, vbp);
+      // (Z G3(nu)) G3(nu')
+      const double2* hrow = H + (size_t)vb * n2 * n2 + p * n2;
+      const double2* gcol = g3q + (size_t)vc * n2 * n2;
+      double2 f2 = make_double2(0.0, 0.0);
+      for (int u = 0; u < n2; ++u) cfma(f2, hrow[u], gcol[u * n2 + sidx]);
+      o[(size_t)row * Mb + sidx * nvp + vbp] = cadd(f1, f2);
     }
+    __syncthreads();
     if (tid == 0 && status) status[item] = singular ? DGA_ITEM_SINGULAR : 0;
     __syncthreads();
   }
@@ -983,7 +1074,8 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
 // (LAPACK's pivot order) with one CTA per matrix; the solves spread over (matrix, block of DENSE_RHS right-hand
 // sides) CTAs, each streaming the factors once for its block.
 // ----------------------------------------------------------------------------------------------
-constexpr int DENSE_RHS = 16;
+constexpr int DENSE_RHS = 16;   // right-hand sides are padded to a multiple of this
+constexpr int DENSE_COLS = 64;  // columns a CTA solves: 16 a warp
 
 template <int NT>
 __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
@@ -993,7 +1085,7 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
   Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
   for (int m = blockIdx.x; m < n_mat; m += gridDim.x) {
-    const bool singular = lu_factor_dmma<NT>(a + (size_t)m * mat_stride, N, N, piv, sm.lu);
+    const bool singular = fp64_lu<NT>(a + (size_t)m * mat_stride, N, N, piv, sm);
     __syncthreads();
     for (int i = threadIdx.x; i < N; i += NT) piv_out[(size_t)m * N + i] = piv[i];
     if (threadIdx.x == 0) status[m] = singular ? DGA_ITEM_SINGULAR : DGA_ITEM_OK;
@@ -1017,11 +1109,12 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
   }
 }
 
-// out_m[:, k] = A_m^-1 B_m[:, k] for k < n_rhs, column-major with leading dimension N, in blocks of DENSE_RHS
-// columns (columns n_rhs .. of the last block are solved for zero right-hand sides).  B_m(r, k) =
+// out_m[:, k] = A_m^-1 B_m[:, k] for k < n_rhs, column-major with leading dimension N, DENSE_COLS
+// columns a CTA (columns n_rhs .. of the last 16 are solved for zero right-hand sides): substitution by 32-row blocks, each
+// accumulated on the FP64 tensor pipe over all solved blocks, with the diagonal blocks inverted.  B_m(r, k) =
 // b[m b_sm + r b_sr + k b_sk], or the identity when b is null.  A non-finite solution element sets
 // DGA_ITEM_NONFINITE in status[m].
-__global__ void __launch_bounds__(BSE_THREADS, 3)
+__global__ void __launch_bounds__(BSE_THREADS, fp64_min_blocks(BSE_THREADS))
     dense_solve_kernel(const double2* __restrict__ lu, const int* __restrict__ piv, int N, int n_mat,
                        long long lu_stride, const double2* __restrict__ b, long long b_sm, long long b_sr,
                        long long b_sk, int n_rhs, double2* __restrict__ out, long long out_stride,
@@ -1030,13 +1123,13 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
   Fp64Smem<BSE_THREADS>& sm = *reinterpret_cast<Fp64Smem<BSE_THREADS>*>(smem_raw);
   int* perm = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<BSE_THREADS>));
   const int tid = threadIdx.x, T = blockDim.x;
-  const int n_blk = (n_rhs + DENSE_RHS - 1) / DENSE_RHS;
+  const int cols = (n_rhs + DENSE_RHS - 1) / DENSE_RHS * DENSE_RHS, n_blk = (cols + DENSE_COLS - 1) / DENSE_COLS;
   for (int t = blockIdx.x; t < n_mat * n_blk; t += gridDim.x) {
-    const int m = t / n_blk, k0 = (t - m * n_blk) * DENSE_RHS;
+    const int m = t / n_blk, k0 = (t - m * n_blk) * DENSE_COLS, nc = min(DENSE_COLS, cols - k0);
     const int* pv = piv + (size_t)m * N;
     build_perm(N, pv, perm);
     double2* Y = out + (size_t)m * out_stride + (size_t)k0 * N;
-    for (int e = tid; e < N * DENSE_RHS; e += T) {
+    for (int e = tid; e < N * nc; e += T) {
       const int i = e % N, k = e / N, col = k0 + k;
       double2 v = make_double2(0.0, 0.0);
       if (col < n_rhs) {
@@ -1049,10 +1142,11 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
       Y[(size_t)k * N + i] = v;
     }
     __syncthreads();
-    lu_solve_inplace<double2, double2, DENSE_RHS>(lu + (size_t)m * lu_stride, N, N, Y, sm.solve.L11,
-                                                  sm.solve.yb);
+    const double2* f = lu + (size_t)m * lu_stride;
+    lu_forward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
+    lu_backward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
     int bad = 0;
-    for (int e = tid; e < N * DENSE_RHS; e += T) {
+    for (int e = tid; e < N * nc; e += T) {
       const double2 v = Y[e];
       bad |= !(isfinite(v.x) && isfinite(v.y));
     }
@@ -1069,68 +1163,36 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
 // the three-leg vertex of the whole pass) is added afterwards by eli_ladder_term_kernel; f1 + term is the sum
 // eli_full_vertex_kernel forms, in the same order, from the same factors.
 // ----------------------------------------------------------------------------------------------
-template <int NT>
-__device__ void eli_box_epilogue(const StructuredSource& src, const WorkItem& wi, int N, int n2, int NRB, int nv, int W, int P,
-                                 double beta2, const double2* __restrict__ A, double2* __restrict__ Y,
-                                 const int* __restrict__ perm, double2* __restrict__ o, Fp64Smem<NT>& sm) {
-  const int tid = threadIdx.x, T = blockDim.x;
-  const int nvp = 2 * P, Mb = n2 * nvp, KB = NRB / n2, off = nv / 2 - P;
-  for (int v0 = 0; v0 < nvp; v0 += KB) {
-    for (int e = tid; e < N * NRB; e += T) {
-      const int i = e % N, sidx = e / N;
-      const int kk = sidx / n2, mp = sidx - kk * n2;
-      const int vb = v0 + kk;
-      const int j = mp * nv + off + vb;
-      Y[(size_t)sidx * N + i] = make_double2((kk < KB && vb < nvp && perm[i] == j) ? 1.0 : 0.0, 0.0);
-    }
-    __syncthreads();
-    lu_solve_n2<NT>(NRB, A, N, Y, sm);
-    for (int e = tid; e < Mb * KB * n2; e += T) {
-      const int sidx = e % n2;
-      const int kk = (e / n2) % KB;
-      const int row = e / (n2 * KB);
-      const int vbp = v0 + kk;
-      if (vbp >= nvp) continue;
-      const int p = row / nvp, vb = row - p * nvp;
-      const int vr = off + vb, vc = off + vbp;
-      const double2* c0r = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vr) * n2 * n2;
-      const double2* c0c = src.chi0_inv + (((size_t)wi.q * W + wi.w) * nv + vc) * n2 * n2;
-      double2 t = make_double2(0.0, 0.0);
-      for (int m = 0; m < n2; ++m) {
-        double2 inner = make_double2(0.0, 0.0);
-        for (int mp = 0; mp < n2; ++mp) cfma(inner, Y[(size_t)(kk * n2 + mp) * N + m * nv + vr], c0c[mp * n2 + sidx]);
-        cfma(t, c0r[p * n2 + m], inner);
-      }
-      double2 f1 = make_double2(-t.x, -t.y);
-      if (vb == vbp) f1 = cadd(f1, c0r[p * n2 + sidx]);
-      o[(size_t)row * Mb + sidx * nvp + vbp] = cscale(f1, beta2);
-    }
-    __syncthreads();
-  }
-}
-
-// FP64 BSE (as bse_solve_sum_fp64_kernel) with the pp-box epilogue for items w < Wpp; NRB = box columns per solve
-// (KB = NRB / n2 box frequencies).  out_pp: [2][Q][Wpp][Mb][Mb].
+// FP64 BSE (as bse_solve_sum_fp64_kernel) with the pp-box epilogue for items w < Wpp.  out_pp: [2][Q][Wpp][Mb][Mb].
 template <int NT>
 __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
     bse_fp64_eli_kernel(StructuredSource src, const WorkItem* __restrict__ work, int n_items, int N, int n2, int nv,
-                        int W, int Q, double beta, double2* __restrict__ out, int NRB, int P, int Wpp,
+                        int W, int Q, double beta, double2* __restrict__ out, int P, int Wpp,
                         double2* __restrict__ out_pp, int* __restrict__ status, double2* __restrict__ scratch,
                         size_t slot_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Fp64Smem<NT>& sm = *reinterpret_cast<Fp64Smem<NT>*>(smem_raw);
   int* piv = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<NT>));
-  int* perm = piv + N;
   double2* A = scratch + (size_t)blockIdx.x * slot_elems;
-  double2* Y = A + (size_t)N * N;
-  const int Mb = n2 * 2 * P;
+  double2* Y = A + (size_t)N * (N + n2);
+  const int nvp = 2 * P, Mb = n2 * nvp;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const WorkItem wi = work[item];
     double2* o = out + (((size_t)wi.ch * Q + wi.q) * W + wi.w) * (size_t)N * n2;
-    const int st = solve_item_fp64<StructuredSource, NT>(src, wi, N, n2, nv, beta, o, A, Y, sm, piv, perm);
-    if (wi.w < Wpp) {
+    const bool box = wi.w < Wpp;
+    if (box) eli_box_columns(N, n2, nv, P, Y);
+    const int st =
+        solve_item_fp64<StructuredSource, NT>(src, wi, N, n2, nv, beta, o, A, sm, piv, box ? Mb : 0);
+    if (box) {
+      fp64_backward<NT>(A, N, Y, Mb, sm);
       double2* opp = out_pp + (((size_t)wi.ch * Q + wi.q) * Wpp + wi.w) * (size_t)Mb * Mb;
-      eli_box_epilogue<NT>(src, wi, N, n2, NRB, nv, W, P, beta * beta, A, Y, perm, opp, sm);
+      for (int e = threadIdx.x; e < Mb * Mb; e += NT) {
+        const int sidx = e % n2, vbp = (e / n2) % nvp, row = e / Mb;
+        const int p = row / nvp, vb = row - p * nvp;
+        opp[(size_t)row * Mb + sidx * nvp + vbp] =
+            eli_box_element(src, wi, W, n2, nv, N, nv / 2 - P, P, beta * beta, Y, p, vb, sidx, vbp);
+      }
+      __syncthreads();
     }
     if (threadIdx.x == 0 && status) status[item] = st;
   }
@@ -1187,39 +1249,42 @@ __global__ void eli_ladder_term_kernel(const double2* __restrict__ uv, const dou
 
 using namespace dga;
 
-// Dynamic shared memory of an FP64 kernel for sizes up to N.
-static size_t bse_smem_bytes(int N) {
-  const int nt = fp64_threads(N);
-  const size_t s = nt == 64 ? sizeof(Fp64Smem<64>) : nt == 128 ? sizeof(Fp64Smem<128>) : sizeof(Fp64Smem<256>);
-  return s + 2 * sizeof(int) * (size_t)N;
-}
-
-// Calls f with the FP64 kernels' thread count for sizes up to N as a compile-time constant.
+// Calls f with the FP64 kernels' thread count for n_items items of sizes up to N as a compile-time constant, and their
+// dynamic shared memory.
 template <typename F>
-static auto with_fp64_threads(int N, F f) {
-  switch (fp64_threads(N)) {
-    case 64: return f(std::integral_constant<int, 64>{});
-    case 128: return f(std::integral_constant<int, 128>{});
-    default: return f(std::integral_constant<int, 256>{});
+static auto with_fp64_threads(int N, int n_items, F f) {
+  const size_t piv = sizeof(int) * (size_t)N;
+  switch (fp64_threads(N, n_items)) {
+    case 32: return f(std::integral_constant<int, 32>{}, sizeof(Fp64Smem<32>) + piv);
+    case 64: return f(std::integral_constant<int, 64>{}, sizeof(Fp64Smem<64>) + piv);
+    case 128: return f(std::integral_constant<int, 128>{}, sizeof(Fp64Smem<128>) + piv);
+    default: return f(std::integral_constant<int, 256>{}, sizeof(Fp64Smem<256>) + piv);
   }
 }
 
+// Resident CTAs of the kernel per SM at this much dynamic shared memory, with the kernel's limits set for it. Without the
+// carve-out the driver may size shared memory for fewer CTAs than fit (six of eight for the two-warp FP64 kernel).
 template <typename K>
-static int grid_for(K kernel, int n_items, size_t smem, int threads = BSE_THREADS) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+static int prepare_kernel(K kernel, size_t smem, int threads) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (per_sm < 1) per_sm = 1;
-  int g = sms * per_sm;
+  const size_t used = (size_t)per_sm * (smem + 1024);  // 1 KB of each CTA is the system's
+  const int percent = (int)((used * 100 + 228 * 1024 - 1) / (228 * 1024));
+  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent < 100 ? percent : 100);
+  return per_sm;
+}
+
+template <typename K>
+static int grid_for(K kernel, int n_items, size_t smem, int threads = BSE_THREADS) {
+  const int g = device_sm_count() * prepare_kernel(kernel, smem, threads);
   return n_items < g ? n_items : g;
 }
 
 static int bse_grid(int N, int n_items) {
-  return with_fp64_threads(N, [&](auto nt) {
-    return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  return with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
+    return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, nt.value>, n_items, smem, nt.value);
   });
 }
 
@@ -1229,10 +1294,9 @@ template <typename Source>
 static void launch_fp64(int n2, int grid, cudaStream_t stream, const Source& src, const WorkItem* work, int n_items,
                         int N, int nv, int W, int Q, double beta, double2* out, int* status, double2* scratch,
                         size_t slot, int redo) {
-  const size_t smem = bse_smem_bytes(N);
-  with_fp64_threads(N, [&](auto nt) {
+  with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
     auto kernel = bse_solve_sum_fp64_kernel<Source, nt.value>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    prepare_kernel(kernel, smem, nt.value);
     kernel<<<grid, nt.value, smem, stream>>>(src, work, n_items, N, n2, nv, W, Q, beta, out, status, scratch, slot,
                                              redo);
   });
@@ -1488,16 +1552,14 @@ int dga_bse_solve_sum_mixed_c128(int n_orb, int niv, int niw_half, int n_q, int 
 // ------------------------------------------------------------------------------------------------
 // Eliashberg full vertex (host side)
 // ------------------------------------------------------------------------------------------------
-static int eli_rhs(int n2) { return n2 == 9 ? 9 : 16; }
-
 static int eli_vertex_grid(int N, int n_items) {
-  return with_fp64_threads(N, [&](auto nt) {
-    return grid_for(eli_full_vertex_kernel<nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  return with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
+    return grid_for(eli_full_vertex_kernel<nt.value>, n_items, smem, nt.value);
   });
 }
 
 static size_t eli_slot_elems(int N, int n2, int P) {
-  return (size_t)N * N + (size_t)N * eli_rhs(n2) + (size_t)2 * P * n2 * n2 + (size_t)n2 * n2;
+  return (size_t)N * N + (size_t)N * 2 * P * n2 + (size_t)2 * P * n2 * n2 + (size_t)n2 * n2;
 }
 
 extern "C" {
@@ -1524,8 +1586,6 @@ int dga_eli_full_vertex_c128(int n_orb, int niv, int niw_half, int n_q, int niv_
     dga_set_error("dga_eli_full_vertex_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  const int NR = eli_rhs(n2);
   const int grid = eli_vertex_grid(N, n_items);
   const size_t slot = eli_slot_elems(N, n2, niv_pp);
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
@@ -1541,9 +1601,9 @@ int dga_eli_full_vertex_c128(int n_orb, int niv, int niw_half, int n_q, int niv_
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  with_fp64_threads(N, [&](auto nt) {
+  with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
     eli_full_vertex_kernel<nt.value><<<grid, nt.value, smem, stream>>>(
-        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, niv_pp, w_pp, beta, NR, (const double2*)g3,
+        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, niv_pp, w_pp, beta, (const double2*)g3,
         (const double2*)chi_phys, (double2*)out, status, (double2*)scratch, slot);
   });
   cudaError_t err = cudaGetLastError();
@@ -1605,14 +1665,15 @@ static bool batch_dims(const dga_bse_problem* probs, int n_prob, int mixed, int*
 }
 
 static size_t batch_smem(int n_max, int n2, int mixed) {
-  return mixed ? mixed_smem_bytes(n_max, n2) : bse_smem_bytes(n_max);
+  return mixed ? mixed_smem_bytes(n_max, n2) : 0;  // the FP64 kernels' own: with_fp64_threads
 }
 
 // The batch kernels' grids for requests of sizes up to n_max (n2 = 0: of several orbital counts).
 static int batch_grid(int mixed, int n2, int n_max, int n_items, size_t smem) {
   if (!mixed)
-    return with_fp64_threads(
-        n_max, [&](auto nt) { return grid_for(bse_multi_fp64_kernel<nt.value>, n_items, smem, nt.value); });
+    return with_fp64_threads(n_max, n_items, [&](auto nt, size_t smem64) {
+      return grid_for(bse_multi_fp64_kernel<nt.value>, n_items, smem64, nt.value);
+    });
   switch (n2) {
     case 0: return grid_for(bse_multi_mixed_kernel<0>, n_items, smem);
     case 1: return grid_for(bse_multi_mixed_kernel<1>, n_items, smem);
@@ -1711,8 +1772,8 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
       case 16: go(bse_multi_mixed_kernel<16>); break;
     }
   } else {
-    with_fp64_threads(n_max, [&](auto nt) {
-      bse_multi_fp64_kernel<nt.value><<<grid, nt.value, smem, stream>>>(pd, wk, n_items, n_max, status, iters, sc, slot,
+    with_fp64_threads(n_max, n_items, [&](auto nt, size_t smem64) {
+      bse_multi_fp64_kernel<nt.value><<<grid, nt.value, smem64, stream>>>(pd, wk, n_items, n_max, status, iters, sc, slot,
                                                                         redo);
     });
   }
@@ -1777,7 +1838,7 @@ static int tuned_grid(int kernel, int mixed, int N, int n2, int n_items, const d
     *slot = mixed_slot_bytes(N, n2);
     grid = mixed_grid(n_items, *smem);
   } else {
-    *smem = bse_smem_bytes(N);
+    *smem = 0;  // with_fp64_threads
     *slot = ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
     grid = bse_grid(N, n_items);
   }
@@ -1980,8 +2041,7 @@ int dga_lu_batched_c128(void* a, int N, int n_mat, long long mat_stride, int* pi
     return DGA_ERR_ARG;
   }
   if (N <= LU_MAX_N) {
-    const size_t smem = bse_smem_bytes(N);
-    with_fp64_threads(N, [&](auto nt) {
+    with_fp64_threads(N, n_mat, [&](auto nt, size_t smem) {
       const int grid = grid_for(dense_lu_kernel<nt.value>, n_mat, smem, nt.value);
       dense_lu_kernel<nt.value><<<grid, nt.value, smem, stream>>>((double2*)a, N, n_mat, mat_stride, piv, status);
     });
@@ -2009,7 +2069,7 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
     return DGA_ERR_ARG;
   }
   const size_t smem = sizeof(Fp64Smem<BSE_THREADS>) + sizeof(int) * (size_t)N;
-  const long long n_tasks = (long long)n_mat * (cols / DENSE_RHS);
+  const long long n_tasks = (long long)n_mat * ((cols + DENSE_COLS - 1) / DENSE_COLS);
   if (n_tasks > 0x7fffffffLL) {
     dga_set_error("dga_lu_solve_batched_c128: too many right-hand-side blocks");
     return DGA_ERR_ARG;
@@ -2028,9 +2088,12 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
 
 }  // extern "C"
 
+// Scratch of one CTA of the fused form: the matrix, the selectors and the box columns, at most N of them (niv_pp <= niv).
+static size_t eli_fused_slot(int N, int n2) { return (size_t)N * N + (size_t)N * n2 + (size_t)N * N; }
+
 static int eli_grid(int N, int n_items) {
-  return with_fp64_threads(N, [&](auto nt) {
-    return grid_for(bse_fp64_eli_kernel<nt.value>, n_items, bse_smem_bytes(N), nt.value);
+  return with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
+    return grid_for(bse_fp64_eli_kernel<nt.value>, n_items, smem, nt.value);
   });
 }
 
@@ -2040,7 +2103,7 @@ extern "C" {
 size_t dga_bse_eli_scratch_bytes(int N, int n2, int n_items) {
   if (N <= 0 || !supported_rhs(n2) || n_items <= 0) return 0;
   const int grid = eli_grid(N, n_items);
-  return (size_t)grid * ((size_t)N * N + (size_t)N * eli_rhs(n2)) * sizeof(double2);
+  return (size_t)grid * eli_fused_slot(N, n2) * sizeof(double2);
 }
 
 // dga_bse_solve_sum_c128 whose items with w < w_pp also write the chi* part of the Eliashberg full vertex in the pp
@@ -2057,8 +2120,7 @@ int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_
     dga_set_error("dga_bse_solve_sum_eli_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const size_t smem = bse_smem_bytes(N);
-  const size_t slot = (size_t)N * N + (size_t)N * eli_rhs(n2);
+  const size_t slot = eli_fused_slot(N, n2);
   const int grid = eli_grid(N, n_items);
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_solve_sum_eli_c128: scratch too small");
@@ -2073,9 +2135,9 @@ int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  with_fp64_threads(N, [&](auto nt) {
+  with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
     bse_fp64_eli_kernel<nt.value><<<grid, nt.value, smem, stream>>>(
-        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, beta, (double2*)out, eli_rhs(n2), niv_pp, w_pp,
+        src, (const WorkItem*)work, n_items, N, n2, nv, niw_half, n_q, beta, (double2*)out, niv_pp, w_pp,
         (double2*)out_pp, status, (double2*)scratch, slot);
   });
   cudaError_t err = cudaGetLastError();

@@ -14,10 +14,11 @@
 // interleaved complex matrix are one 16-byte load per lane each (lane (g, t) holds row g and column t), so operands come
 // straight from L2 and L1: four warps per SM already reach 35 TFLOP/s. The tcgen05 pipe has no FP64 kind.
 //
-// What bounds it: the products at N = 720 (592 factorisations in 27.0 ms, 21.9 TFLOP/s, two CTAs an SM, three quarters of
-// the time in the block columns and rows), the panels' dependent steps below about N = 200 (14,208 of N = 120 in 7.9 ms).
-// Whole passes, from the right-looking vector-pipe form to this one: 1,130 to 762 ms for three orbitals on 32 x 32
-// (N = 720), 103 to 72 ms for one orbital on 64 x 64 (N = 120), 0.85 to 0.62 ms on 16 x 16 (N = 40).
+// What bounds it: the products at N = 720 (592 factorisations in 27.7 ms, 21.3 TFLOP/s, two CTAs an SM), waits on HBM and
+// L2 for the panels and the tiles' first elements below about N = 250 (14,208 of N = 120 in 7.6 ms, 8.7 TFLOP/s, 45% of the
+// warps' stalls). Whole passes, from the right-looking vector-pipe form to this one: 1,130 to 742 ms for three orbitals on
+// 32 x 32 (N = 720), 103 to 66 ms for one orbital on 64 x 64 (N = 120), 0.84 to 0.41 ms on 16 x 16 (N = 40), 404 to 165 ms
+// for the bilayer on 48 x 48 with its pairing box (N = 240, 124 right-hand sides).
 #pragma once
 
 #include "dga_common.cuh"
@@ -25,10 +26,16 @@
 
 namespace dga {
 
-constexpr int LU_NB = 32;   // block width
 constexpr int LU_MAX_N = 2048;
 constexpr int LU_RING = 4;  // steps of four columns a lane has in flight
-static_assert(LU_RING * 2 == 8, "a warp's ring and its 8-column tile share their memory");
+
+// Block width by the matrix size alone, so that a matrix goes through the same operations whatever CTA it is given. 16 up
+// to N = 192, where one or two warps take a matrix and 16 or 8 matrices share an SM (the shared memory of a 32-wide block
+// would admit five): the panels' chains of dependent steps, not the products, are what the time goes to. 29,600
+// factorisations of N = 40 took 1.71 ms against 2.90 at 32 wide, 9,472 of N = 160 8.7 against 9.2, each with its best
+// thread count; with many right-hand sides the wider block is the faster one from N = 240 (154 against 162 ms for the
+// bilayer pass with its pairing box).
+constexpr int LU_SMALL_N = 192;
 
 // Rows a thread holds in the panel and panel columns it keeps in registers, for matrices of up to RPT * NT rows: at most
 // RPT * PW = 16 complex values (64 registers).
@@ -37,18 +44,20 @@ struct LuPanelWidth {
   static constexpr int value = RPT <= 2 ? 8 : RPT <= 4 ? 4 : 2;
 };
 
-template <int NT>
+constexpr int LU_WARP_BUF = LU_RING * 2 * 33;
+
+template <int NT, int NB>
 struct LuSmem {
-  double2 L11i[LU_NB][LU_NB + 1];  // inverse of the diagonal block's unit lower triangle
+  double2 L11i[NB][NB + 1];  // inverse of the diagonal block's triangle
   union {
-    double2 L11[LU_NB][LU_NB + 1];                    // the triangle itself, dead once it is inverted
-    // (each warp's part is the same memory in both)
-    double2 tile[NT / 32][8][LU_NB + 1];              // per warp: 8 columns of the block row before the triangular solve
-    double2 ring[NT / 32][LU_RING][2][LU_NB + 1];     // per lane: fragments of the streamed factor on their way from HBM
+    double2 L11[NB][NB + 1];  // the triangle itself, dead once it is inverted
+    // per warp: each lane's fragments of the streamed factor on their way from HBM ([LU_RING][2][33]), then 8 columns of the
+    // block row before the triangular solve ([8][NB + 1])
+    double2 warp[NT / 32][LU_WARP_BUF];
   };
-  double2 us[8][LU_NB];            // panel: rows of U of the columns just factored
+  double2 us[8][NB];               // panel: rows of U of the columns just factored
   double2 cand[2][NT / 32][10];    // panel: each warp's candidate pivot row, conj(pivot), 1 / |pivot|^2
-  __align__(16) unsigned long long key[2][NT / 32];
+  __align__(16) unsigned long long key[2][(NT / 32 + 1) / 2 * 2];
   int flag;
 };
 
@@ -56,6 +65,13 @@ __device__ __forceinline__ void cp_async16(double2* smem, const double2* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
                : "memory");
 }
+// fill: 16 bytes of zeros in place of the source where false
+__device__ __forceinline__ void cp_async16_or_zero(double2* smem, const double2* g, bool fill) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g),
+               "r"(fill ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void prefetch_l1(const double2* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -74,6 +90,12 @@ struct CAcc {
   double re[4], im[4];
 };
 
+// a b with one rounding order everywhere: left to the compiler, the contraction may differ between kernels that must give
+// the same bits
+__device__ __forceinline__ double2 cmul_fma(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+
 // c[n] += a b[n] on complex fragments: the products with Re a first, then those with Im a (one negated copy)
 template <int NTILE>
 __device__ __forceinline__ void cdmma_row(CAcc* c, double2 a0, double2 a1, const double2* b) {
@@ -90,37 +112,40 @@ __device__ __forceinline__ void cdmma_row(CAcc* c, double2 a0, double2 a1, const
   }
 }
 
-// Block column: A[j0.., j0 .. j0+nb) -= A[j0.., 0..j0) A[0..j0, j0 .. j0+nb). One warp per 16 rows x 32 columns; rows and
+// Block column: A[j0.., j0 .. j0+nb) -= A[j0.., 0..j0) A[0..j0, j0 .. j0+nb). One warp per 16 rows x NB columns; rows and
 // columns past the end read the last valid ones and are not stored. L streams from HBM (the matrices in flight are ten
-// times L2): a lane copies the two elements it multiplies three steps later, 1,500 cycles of the FP64 pipe, into its own
+// times L2): a lane copies the two elements it multiplies three steps later, 1,500 cycles of the FP64 pipe at NB = 32, into its own
 // ring slot, so nothing has to be synchronised; U is shared by all warps and comes from L1, one step ahead.
-template <int NT>
-__device__ void lu_block_column(double2* __restrict__ A, int N, int ld, int j0, int nb, LuSmem<NT>& sm) {
+template <int NT, int NB>
+__device__ void lu_block_column(double2* __restrict__ A, int N, int ld, int j0, int nb, LuSmem<NT, NB>& sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int tiles = (N - j0 + 15) / 16;
-  double2(*ring)[2][LU_NB + 1] = sm.ring[warp];
-  int ob[4];
+  double2(*ring)[2][33] = reinterpret_cast<double2(*)[2][33]>(sm.warp[warp]);
+  constexpr int NTN = NB / 8;
+  int ob[NTN];
 #pragma unroll
-  for (int nt = 0; nt < 4; ++nt) ob[nt] = min(j0 + nt * 8 + g, N - 1) * ld + t;
+  for (int nt = 0; nt < NTN; ++nt) ob[nt] = min(j0 + nt * 8 + g, N - 1) * ld + t;
   for (int tile = warp; tile < tiles; tile += NT / 32) {
     const int r0 = j0 + tile * 16 + g, r1 = r0 + 8;
-    CAcc acc[4];
+    CAcc acc[NTN];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < NTN; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[nt].re[i] = acc[nt].im[i] = 0.0;
     const int d1 = min(r1, N - 1) - min(r0, N - 1), step = 4 * ld;
     const double2* pa = A + t * ld + min(r0, N - 1);
+    // the tile itself, read after the products: 256 bytes a column, one 128-byte line a lane
+    for (int e = lane; e < 2 * nb; e += 32) prefetch_l1(A + (size_t)(j0 + e / 2) * ld + min(j0 + tile * 16 + (e & 1) * 8, N - 1));
 #pragma unroll
-    for (int u = 0; u < LU_RING - 1; ++u) {  // j0 >= 32: at least eight steps
+    for (int u = 0; u < LU_RING - 1; ++u) {  // j0 >= 16: at least four steps
       cp_async16(&ring[u][0][lane], pa);
       cp_async16(&ring[u][1][lane], pa + d1);
       cp_async_commit();
       pa += step;
     }
-    double2 b[4];
+    double2 b[NTN];
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) b[nt] = A[ob[nt]];
+    for (int nt = 0; nt < NTN; ++nt) b[nt] = A[ob[nt]];
     int slot = 0;
     for (int k = 0; k < j0; k += 4) {
       cp_async_wait<LU_RING - 2>();
@@ -133,17 +158,17 @@ __device__ void lu_block_column(double2* __restrict__ A, int N, int ld, int j0, 
       }
       cp_async_commit();
       slot = (slot + 1) % LU_RING;
-      double2 y[4];
+      double2 y[NTN];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) y[nt] = b[nt];
+      for (int nt = 0; nt < NTN; ++nt) y[nt] = b[nt];
       if (k + 4 < j0) {
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) b[nt] = A[ob[nt] + k + 4];
+        for (int nt = 0; nt < NTN; ++nt) b[nt] = A[ob[nt] + k + 4];
       }
-      cdmma_row<4>(acc, x0, x1, y);
+      cdmma_row<NTN>(acc, x0, x1, y);
     }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < NTN; ++nt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int c = nt * 8 + 2 * t + (i & 1), r = i < 2 ? r0 : r1;
@@ -155,88 +180,106 @@ __device__ void lu_block_column(double2* __restrict__ A, int N, int ld, int j0, 
   }
 }
 
-// Block row: U[j0..j0+32, c] = L11^-1 (A[j0..j0+32, c] - A[j0..j0+32, 0..j0) A[0..j0, c]) for the columns c >= j0 + 32.
-// One warp per 32 rows x 16 columns; the triangular solve is a product with the inverse in shared memory.
-template <int NT>
-__device__ void lu_block_row(double2* __restrict__ A, int N, int ld, int j0, LuSmem<NT>& sm) {
+// Block row of ncols columns Y (leading dimension ldy; the matrix's own to the right of the block, or right-hand sides):
+//   Y[j0..j0+nb) = T^-1 (Y[j0..j0+nb) - A[j0..j0+nb, k0..k1) Y[k0..k1)),   T^-1 in sm.L11i.
+// UPPER false: T = L11, k0 = 0, k1 = j0 (the factorisation's block row, forward substitution); UPPER true: T = U11,
+// k0 = j0 + nb, k1 = N (backward substitution). One warp per NB rows x 16 columns: Y streams through the ring, the rows of
+// A are shared by all warps and come from L1. Rows past nb count as zero, columns past ncols read the last one and are
+// not stored.
+template <int NT, int NB, bool UPPER>
+__device__ void lu_block_row(const double2* __restrict__ A, int N, int ld, int j0, int nb, int k0, int k1, double2* Y,
+                             int ldy, int ncols, LuSmem<NT, NB>& sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int c_first = j0 + LU_NB, tiles = (N - c_first + 15) / 16;
+  constexpr int MT = NB / 16;
+  const int tiles = (ncols + 15) / 16, steps = (k1 - k0 + 3) / 4;
   for (int tile = warp; tile < tiles; tile += NT / 32) {
-    const int c0 = c_first + tile * 16;
-    CAcc acc[2][2];  // [16-row half][8-column half]
+    const int c0 = tile * 16;
+    CAcc acc[MT][2];  // [16-row half][8-column half]
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[mt][nt].re[i] = acc[mt][nt].im[i] = 0.0;
-    if (j0 > 0) {
-      double2(*ring)[2][LU_NB + 1] = sm.ring[warp];
-      int oa = t * ld + j0 + g;
-      const double2* pb = A + (size_t)min(c0 + g, N - 1) * ld + t;
-      const int d1 = (min(c0 + 8 + g, N - 1) - min(c0 + g, N - 1)) * ld, step = 4 * ld;
+    if (steps > 0) {
+      double2(*ring)[2][33] = reinterpret_cast<double2(*)[2][33]>(sm.warp[warp]);
+      const double2* pb = Y + (size_t)min(c0 + g, ncols - 1) * ldy + k0 + t;
+      const size_t d1 = (size_t)(min(c0 + 8 + g, ncols - 1) - min(c0 + g, ncols - 1)) * ldy;
+      int left = k1 - k0 - t;  // rows of Y from this lane's on; past the end they count as zero
       __syncwarp();  // the ring shares its memory with the previous tile's columns
 #pragma unroll
       for (int u = 0; u < LU_RING - 1; ++u) {
-        cp_async16(&ring[u][0][lane], pb);
-        cp_async16(&ring[u][1][lane], pb + d1);
+        const bool in = left > 0;
+        cp_async16_or_zero(&ring[u][0][lane], in ? pb : Y, in);
+        cp_async16_or_zero(&ring[u][1][lane], in ? pb + d1 : Y, in);
         cp_async_commit();
         pb += 4;
+        left -= 4;
       }
-      double2 a[4];
+      int ra[2 * MT], ca = k0 + t;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = A[oa + u * 8];
+      for (int u = 0; u < 2 * MT; ++u) ra[u] = min(j0 + g + u * 8, N - 1);
+      double2 a[2 * MT];
+#pragma unroll
+      for (int u = 0; u < 2 * MT; ++u) a[u] = A[min(ca, N - 1) * ld + ra[u]];
       int slot = 0;
-      for (int k = 0; k < j0; k += 4) {
+      for (int s = 0; s < steps; ++s) {
         cp_async_wait<LU_RING - 2>();
         const double2 y[2] = {ring[slot][0][lane], ring[slot][1][lane]};
         const int next = (slot + LU_RING - 1) % LU_RING;
-        if (k + 4 * (LU_RING - 1) < j0) {
-          cp_async16(&ring[next][0][lane], pb);
-          cp_async16(&ring[next][1][lane], pb + d1);
+        if (s + LU_RING - 1 < steps) {
+          const bool in = left > 0;
+          cp_async16_or_zero(&ring[next][0][lane], in ? pb : Y, in);
+          cp_async16_or_zero(&ring[next][1][lane], in ? pb + d1 : Y, in);
           pb += 4;
+          left -= 4;
         }
         cp_async_commit();
         slot = (slot + 1) % LU_RING;
-        double2 x[4];
+        double2 x[2 * MT];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = a[u];
-        if (k + 4 < j0) {
-          oa += step;
+        for (int u = 0; u < 2 * MT; ++u) x[u] = a[u];
+        if (s + 1 < steps) {
+          ca += 4;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) a[u] = A[oa + u * 8];
+          for (int u = 0; u < 2 * MT; ++u) a[u] = A[min(ca, N - 1) * ld + ra[u]];
         }
-        cdmma_row<2>(acc[0], x[0], x[1], y);
-        cdmma_row<2>(acc[1], x[2], x[3], y);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) cdmma_row<2>(acc[mt], x[2 * mt], x[2 * mt + 1], y);
       }
     }
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
-      double2(&w)[8][LU_NB + 1] = sm.tile[warp];
+      double2(*w)[NB + 1] = reinterpret_cast<double2(*)[NB + 1]>(sm.warp[warp]);
       __syncwarp();
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int c = min(c0 + nt * 8 + 2 * t + (i & 1), N - 1), r = mt * 16 + g + (i < 2 ? 0 : 8);
-          const double2 v = A[(size_t)c * ld + j0 + r];
-          w[2 * t + (i & 1)][r] = make_double2(v.x - acc[mt][nt].re[i], v.y - acc[mt][nt].im[i]);
+          const int c = min(c0 + nt * 8 + 2 * t + (i & 1), ncols - 1), r = mt * 16 + g + (i < 2 ? 0 : 8);
+          double2 v = make_double2(0.0, 0.0);
+          if (r < nb) {
+            v = Y[(size_t)c * ldy + j0 + r];
+            v = make_double2(v.x - acc[mt][nt].re[i], v.y - acc[mt][nt].im[i]);
+          }
+          w[2 * t + (i & 1)][r] = v;
         }
       __syncwarp();
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         CAcc x[1];
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[0].re[i] = x[0].im[i] = 0.0;
+        const int from = UPPER ? mt * 16 : 0, to = UPPER ? NB : mt * 16 + 16;
 #pragma unroll 2
-        for (int k = 0; k < mt * 16 + 16; k += 4) {
+        for (int k = from; k < to; k += 4) {
           const double2 y[1] = {w[g][k + t]};
           cdmma_row<1>(x, sm.L11i[mt * 16 + g][k + t], sm.L11i[mt * 16 + g + 8][k + t], y);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int c = c0 + nt * 8 + 2 * t + (i & 1), r = j0 + mt * 16 + g + (i < 2 ? 0 : 8);
-          if (c < N) A[(size_t)c * ld + r] = make_double2(x[0].re[i], x[0].im[i]);
+          const int c = c0 + nt * 8 + 2 * t + (i & 1), r = mt * 16 + g + (i < 2 ? 0 : 8);
+          if (c < ncols && r < nb) Y[(size_t)c * ldy + j0 + r] = make_double2(x[0].re[i], x[0].im[i]);
         }
       }
     }
@@ -253,30 +296,6 @@ __device__ __forceinline__ double2 cdot4(int n, FA a, FB b) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) cfma(s[u], a(k + u), b(k + u));
   return cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
-}
-
-// Inverse of the unit lower 32 x 32 block in sm.L11 by doubling, from the inverses of its 8 x 8 diagonal blocks in
-// sm.L11i: [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1 C^-1] at 16 and 32.
-template <int NT>
-__device__ void lu_unit_lower_inverse(LuSmem<NT>& sm) {
-  const int tid = threadIdx.x;
-  double2* tmp = &sm.us[0][0];  // B A^-1, at most 16 x 16
-#pragma unroll
-  for (int h = 8; h <= 16; h *= 2) {
-    const int n = LU_NB / 2 * h;
-    for (int e = tid; e < n; e += NT) {
-      const int b = e / (h * h), r = (e / h) % h, c = e % h, o = b * 2 * h;
-      tmp[e] = cdot4(h, [&](int k) { return sm.L11[o + h + r][o + k]; }, [&](int k) { return sm.L11i[o + k][o + c]; });
-    }
-    __syncthreads();
-    for (int e = tid; e < n; e += NT) {
-      const int b = e / (h * h), r = (e / h) % h, c = e % h, o = b * 2 * h;
-      const double2 v = cdot4(h, [&](int k) { return sm.L11i[o + h + r][o + h + k]; },
-                              [&](int k) { return tmp[b * h * h + k * h + c]; });
-      sm.L11i[o + h + r][o + c] = make_double2(-v.x, -v.y);
-    }
-    __syncthreads();
-  }
 }
 
 constexpr unsigned long long LU_INF_BITS = 0x7ff0000000000000ull;
@@ -315,18 +334,57 @@ __device__ __forceinline__ void pivot_recip(double2 d, double2& c, double& s) {
   }
 }
 
-// y = L^-1 y for the leading n x n unit lower triangle at L in sm.L11's row pitch; a rotating loop, as in the panel
-template <int PW>
+// y = L^-1 y for the leading n x n unit lower triangle at L (row pitch LD); a rotating loop, as in the panel
+template <int PW, int LD>
 __device__ __forceinline__ void unit_lower_solve(double2 (&y)[PW], int n, const double2* L) {
 #pragma unroll 1
   for (int k = 0; k < PW; ++k) {
     const double2 yk = y[0];
 #pragma unroll
     for (int r = 1; r < PW; ++r)
-      if (k + r < n) cfms(y[r], L[(k + r) * (LU_NB + 1) + k], yk);
+      if (k + r < n) cfms(y[r], L[(k + r) * LD + k], yk);
 #pragma unroll
     for (int r = 0; r + 1 < PW; ++r) y[r] = y[r + 1];
     y[PW - 1] = yk;
+  }
+}
+
+// sm.L11i = inverse of the unit lower NB x NB block in sm.L11 by doubling: its 8 x 8 diagonal blocks by substitution (one
+// thread per column), then [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1 C^-1] at 16 (and 32).
+template <int NT, int NB>
+__device__ void lu_unit_lower_inverse(LuSmem<NT, NB>& sm) {
+  const int tid = threadIdx.x;
+  for (int e = tid; e < NB * NB; e += NT) {
+    const int r = e % NB, c = e / NB;
+    if ((r ^ c) & ~7) sm.L11i[r][c] = make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  if (tid < NB) {
+    const int o = tid & ~7, c = tid & 7;
+    double2 y[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) y[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+    unit_lower_solve<8, NB + 1>(y, 8, &sm.L11[o][o]);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) sm.L11i[o + r][o + c] = y[r];
+  }
+  __syncthreads();
+  double2* tmp = &sm.us[0][0];  // B A^-1, at most 16 x 16
+#pragma unroll
+  for (int h = 8; h < NB; h *= 2) {
+    const int n = NB / 2 * h;
+    for (int e = tid; e < n; e += NT) {
+      const int b = e / (h * h), r = (e / h) % h, c = e % h, o = b * 2 * h;
+      tmp[e] = cdot4(h, [&](int k) { return sm.L11[o + h + r][o + k]; }, [&](int k) { return sm.L11i[o + k][o + c]; });
+    }
+    __syncthreads();
+    for (int e = tid; e < n; e += NT) {
+      const int b = e / (h * h), r = (e / h) % h, c = e % h, o = b * 2 * h;
+      const double2 v = cdot4(h, [&](int k) { return sm.L11i[o + h + r][o + h + k]; },
+                              [&](int k) { return tmp[b * h * h + k * h + c]; });
+      sm.L11i[o + h + r][o + c] = make_double2(-v.x, -v.y);
+    }
+    __syncthreads();
   }
 }
 
@@ -336,9 +394,9 @@ __device__ __forceinline__ void unit_lower_solve(double2 (&y)[PW], int n, const 
 // reciprocal already taken, every thread picks the winner. The PW columns are then applied to the rest of the block, whose
 // interchanges are made here; the columns outside it follow in lu_interchange. Returns true if
 // an exact zero pivot was met.
-template <int NT, int RPT>
+template <int NT, int NB, int RPT>
 __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb, int* __restrict__ piv,
-                         LuSmem<NT>& sm) {
+                         LuSmem<NT, NB>& sm) {
   constexpr int PW = LuPanelWidth<RPT>::value, NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool singular = false;
@@ -427,7 +485,7 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
           else if (pos[i] == j)
             pos[i] = p;
           if (pos[i] > j && pos[i] < N) {
-            if (!zero) a[i][0] = cscale(cmul(a[i][0], cd), cs);
+            if (!zero) a[i][0] = cscale(cmul_fma(a[i][0], cd), cs);
 #pragma unroll
             for (int c = 1; c < PW; ++c)
               if (c < PW - jj) cfms(a[i][c], a[i][0], row[c]);
@@ -477,7 +535,7 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
         double2 y[PW];
 #pragma unroll
         for (int r = 0; r < PW; ++r) y[r] = r < pw ? col[r] : make_double2(0.0, 0.0);
-        unit_lower_solve<PW>(y, pw, &sm.L11[p0][p0]);
+        unit_lower_solve<PW, NB + 1>(y, pw, &sm.L11[p0][p0]);
 #pragma unroll
         for (int r = 0; r < PW; ++r)
           if (r < pw) {
@@ -518,25 +576,38 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
   return singular;
 }
 
-// The unit lower triangle of the factored 32 x 32 diagonal block in sm.L11, and the inverses of its 8 x 8 diagonal blocks
-// (one thread per column) in sm.L11i, zero elsewhere.
-template <int NT>
-__device__ void lu_load_l11(const double2* __restrict__ A, int ld, int j0, LuSmem<NT>& sm) {
+// sm.L11i = L11^-1 of the factored nb x nb diagonal block at j0, as an NB x NB unit lower triangle (identity past nb).
+template <int NT, int NB>
+__device__ void lu_invert_lower(const double2* __restrict__ A, int ld, int j0, int nb, LuSmem<NT, NB>& sm) {
   const int tid = threadIdx.x;
-  for (int e = tid; e < LU_NB * LU_NB; e += NT) {
-    const int r = e % LU_NB, c = e / LU_NB;
-    if (r > c) sm.L11[r][c] = A[(size_t)(j0 + c) * ld + j0 + r];
-    if ((r ^ c) & ~7) sm.L11i[r][c] = make_double2(0.0, 0.0);
+  for (int e = tid; e < NB * NB; e += NT) {
+    const int r = e % NB, c = e / NB;
+    if (r > c) sm.L11[r][c] = r < nb ? A[(size_t)(j0 + c) * ld + j0 + r] : make_double2(0.0, 0.0);
   }
+  lu_unit_lower_inverse<NT, NB>(sm);
+}
+
+// sm.L11i = U11^-1 of the diagonal block (zero past nb): with D its diagonal, U11^-1 = ((D^-1 U11)^T)^-T D^-1, so that the
+// same unit lower inverse serves.
+template <int NT, int NB>
+__device__ void lu_invert_upper(const double2* __restrict__ A, int ld, int j0, int nb, LuSmem<NT, NB>& sm) {
+  const int tid = threadIdx.x;
+  double2* dinv = &sm.cand[0][0][0];
+  if (tid < NB) dinv[tid] = tid < nb ? crecip(A[(size_t)(j0 + tid) * ld + j0 + tid]) : make_double2(0.0, 0.0);
   __syncthreads();
-  if (tid < LU_NB) {
-    const int o = tid & ~7, c = tid & 7;
-    double2 y[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) y[r] = make_double2(r == c ? 1.0 : 0.0, 0.0);
-    unit_lower_solve<8>(y, 8, &sm.L11[o][o]);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) sm.L11i[o + r][o + c] = y[r];
+  for (int e = tid; e < NB * NB; e += NT) {
+    const int c = e % NB, r = e / NB;  // U11[c][r], c < r
+    if (r > c) sm.L11[r][c] = r < nb ? cmul_fma(A[(size_t)(j0 + r) * ld + j0 + c], dinv[c]) : make_double2(0.0, 0.0);
+  }
+  lu_unit_lower_inverse<NT, NB>(sm);
+  for (int e = tid; e < NB * NB; e += NT) {
+    const int i = e % NB, j = e / NB;
+    if (i < j) {
+      sm.L11i[i][j] = cmul_fma(sm.L11i[j][i], dinv[j]);
+      sm.L11i[j][i] = make_double2(0.0, 0.0);
+    } else if (i == j) {
+      sm.L11i[i][i] = dinv[i];
+    }
   }
   __syncthreads();
 }
@@ -544,9 +615,9 @@ __device__ void lu_load_l11(const double2* __restrict__ A, int ld, int j0, LuSme
 // The block's row interchanges on the columns outside it: in parallel over (interchange, column) when they are
 // independent pairs (every pivot row below the block, no two alike), else in order per column; nothing to do when no
 // row moved.
-template <int NT>
-__device__ void lu_interchange(double2* __restrict__ A, int N, int ld, int j0, int nb, const int* __restrict__ piv,
-                               LuSmem<NT>& sm) {
+template <int NT, int NB>
+__device__ void lu_interchange(double2* __restrict__ A, int ncols, int ld, int j0, int nb, const int* __restrict__ piv,
+                               LuSmem<NT, NB>& sm) {
   const int tid = threadIdx.x, k1 = j0 + nb;
   if (tid < 32) {
     bool alone = true, moved = false;
@@ -563,7 +634,7 @@ __device__ void lu_interchange(double2* __restrict__ A, int N, int ld, int j0, i
     if (tid == 0) sm.flag = !any ? 0 : all_alone ? 1 : 2;
   }
   __syncthreads();
-  const int ncol = N - nb;
+  const int ncol = ncols - nb;
   if (sm.flag == 1) {
     for (int jj = 0; jj < nb; ++jj) {
       const int j = j0 + jj, p = piv[j];
@@ -592,33 +663,59 @@ __device__ void lu_interchange(double2* __restrict__ A, int N, int ld, int j0, i
 }
 
 // LU of the N x N column-major matrix A (leading dimension ld) in place, N <= 8 NT and N <= 2048. piv: N entries in shared
-// memory. The result does not depend on NT: every element goes through the same operations in the same order.
-template <int NT>
-__device__ __noinline__ bool lu_factor_dmma(double2* __restrict__ A, int N, int ld, int* __restrict__ piv, LuSmem<NT>& sm) {
+// memory. The columns N .. ncols - 1 are right-hand sides: they take the interchanges and the block rows with the matrix
+// and leave as L^-1 P B, so that only the backward substitution is left. The result does not depend on NT: every element
+// goes through the same operations in the same order.
+template <int NT, int NB>
+__device__ bool lu_factor_dmma(double2* __restrict__ A, int N, int ncols, int ld, int* __restrict__ piv,
+                                            LuSmem<NT, NB>& sm) {
   bool singular = false;
-  for (int j0 = 0; j0 < N; j0 += LU_NB) {
-    const int nb = min(LU_NB, N - j0), m = N - j0;
+  for (int j0 = 0; j0 < N; j0 += NB) {
+    const int nb = min(NB, N - j0), m = N - j0, right = ncols - j0 - nb;
     if (j0 > 0) {
-      lu_block_column<NT>(A, N, ld, j0, nb, sm);
+      lu_block_column<NT, NB>(A, N, ld, j0, nb, sm);
       __syncthreads();
     }
     if (m <= NT)
-      singular |= lu_panel<NT, 1>(A, N, ld, j0, nb, piv, sm);
+      singular |= lu_panel<NT, NB, 1>(A, N, ld, j0, nb, piv, sm);
     else if (m <= 2 * NT)
-      singular |= lu_panel<NT, 2>(A, N, ld, j0, nb, piv, sm);
+      singular |= lu_panel<NT, NB, 2>(A, N, ld, j0, nb, piv, sm);
     else if (m <= 4 * NT)
-      singular |= lu_panel<NT, 4>(A, N, ld, j0, nb, piv, sm);
+      singular |= lu_panel<NT, NB, 4>(A, N, ld, j0, nb, piv, sm);
     else
-      singular |= lu_panel<NT, 8>(A, N, ld, j0, nb, piv, sm);
-    lu_interchange<NT>(A, N, ld, j0, nb, piv, sm);
-    if (j0 + nb < N) {
-      lu_load_l11<NT>(A, ld, j0, sm);
-      lu_unit_lower_inverse<NT>(sm);
-      lu_block_row<NT>(A, N, ld, j0, sm);
+      singular |= lu_panel<NT, NB, 8>(A, N, ld, j0, nb, piv, sm);
+    lu_interchange<NT, NB>(A, ncols, ld, j0, nb, piv, sm);
+    if (right > 0) {
+      lu_invert_lower<NT, NB>(A, ld, j0, nb, sm);
+      lu_block_row<NT, NB, false>(A, N, ld, j0, nb, 0, j0, A + (size_t)(j0 + nb) * ld, ld, right, sm);
       __syncthreads();
     }
   }
   return singular;
+}
+
+// Y = L^-1 Y (rows already interchanged) for the ncols columns of Y, with the factors of lu_factor_dmma.
+template <int NT, int NB>
+__device__ void lu_forward_dmma(const double2* __restrict__ A, int N, int ld, double2* Y, int ldy, int ncols,
+                                             LuSmem<NT, NB>& sm) {
+  for (int j0 = 0; j0 < N; j0 += NB) {
+    const int nb = min(NB, N - j0);
+    lu_invert_lower<NT, NB>(A, ld, j0, nb, sm);
+    lu_block_row<NT, NB, false>(A, N, ld, j0, nb, 0, j0, Y, ldy, ncols, sm);
+    __syncthreads();
+  }
+}
+
+// Y = U^-1 Y for the ncols columns of Y.
+template <int NT, int NB>
+__device__ void lu_backward_dmma(const double2* __restrict__ A, int N, int ld, double2* Y, int ldy,
+                                              int ncols, LuSmem<NT, NB>& sm) {
+  for (int j0 = (N - 1) / NB * NB; j0 >= 0; j0 -= NB) {
+    const int nb = min(NB, N - j0);
+    lu_invert_upper<NT, NB>(A, ld, j0, nb, sm);
+    lu_block_row<NT, NB, true>(A, N, ld, j0, nb, j0 + nb, N, Y, ldy, ncols, sm);
+    __syncthreads();
+  }
 }
 
 }  // namespace dga
