@@ -48,7 +48,7 @@ def up_to_date() -> bool:
 
 
 def _compile_cmd(nvcc: str, src: str, obj: str, ptxas_info: bool) -> list[str]:
-    cmd = [nvcc, *ARCH_FLAGS, "-O3", "-lineinfo", "-std=c++17", "-fmad=true", "-split-compile=0", "-Xcompiler", "-fPIC", "-c",
+    cmd = [nvcc, *ARCH_FLAGS, "-O3", "-lineinfo", "-std=c++17", "-fmad=true", "-Xcompiler", "-fPIC", "-c",
            "-I", os.path.join(os.path.dirname(HERE), "include"), "-o", obj, src]
     if ptxas_info:
         cmd.insert(1, "-Xptxas=-v")
