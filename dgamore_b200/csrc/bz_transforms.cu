@@ -9,9 +9,10 @@
 //                          the irreducible kernel through the IBZ -> FBZ map (n_point_base.py:489-494) and the
 //                          w < 0 half from K(q,-w,nu) = conj K(q,w,-nu-1) (local_n_point.py:191-225).
 //
-// A plane (Nk = nx*ny*nz points, C order) sits in shared memory; each axis is a direct DFT against a
-// host-built FP64 twiddle table (e^{2 pi i m / n}, sign folded in), so the transform needs no FFT plan and
-// handles any grid (16, 32, 48, 64, ...).  Work per plane is Nk*(nx+ny+nz) complex FMAs.
+// A plane (Nk = nx*ny*nz points, C order) sits in shared memory; each axis is a two-stage Cooley-Tukey DFT (J. W. Cooley
+// and J. W. Tukey, Math. Comp. 19, 297 (1965)) against a host-built FP64 twiddle table (e^{2 pi i m / n}, sign folded in),
+// so the transform needs no plan and handles any grid: an axis of n = n1 n2 points, n1 the largest divisor up to sqrt(n),
+// takes n1 + n2 complex FMAs a point (14 instead of 48 at n = 48; a prime n is a direct sum).
 #include "dga_common.cuh"
 
 namespace dga {
@@ -22,99 +23,96 @@ constexpr int BZ_MAX_AXIS = 128;
 
 struct Grid3 {
   int nx, ny, nz, nk;
+  int fx, fy, fz;  // first-stage lengths of the axes' transforms (axis_split)
 };
+
+// Largest divisor of n up to sqrt(n); 1, a direct sum in one stage, up to n = 16, where the second stage's barrier and
+// index arithmetic cost more than the products they save (15.3 against 12.3 us for the three transforms of a 9 x 9 pass).
+inline int axis_split(int n) {
+  int n1 = 1;
+  if (n <= 16) return n1;
+  for (int d = 2; d * d <= n; ++d)
+    if (n % d == 0) n1 = d;
+  return n1;
+}
+
+inline Grid3 make_grid(int nx, int ny, int nz) {
+  return Grid3{nx, ny, nz, nx * ny * nz, axis_split(nx), axis_split(ny), axis_split(nz)};
+}
 
 // twiddle tables in shared memory: tw[0..nx) for x, then y, then z
 __device__ __forceinline__ void load_twiddles(double2* s_tw, const double2* tw, const Grid3 g) {
   for (int i = threadIdx.x; i < g.nx + g.ny + g.nz; i += blockDim.x) s_tw[i] = tw[i];
 }
 
-// DFT along x of an nx x (ny nz) plane in shared memory (in -> out, both [x][yz]; twx = the nx twiddles),
-// followed by a barrier.
-constexpr int XR = 4;  // outputs per thread of the blocked axis passes
-__device__ __forceinline__ void dft_axis_x(const double2* in, double2* out, const double2* twx, const Grid3 g) {
-  const int T = blockDim.x, nyz = g.ny * g.nz;
-  // A thread computes the outputs kx = grp + j ngx (j < XR) of one yz column, so each load serves XR
-  // products (the twiddle loads are warp broadcasts); every output still sums over x in order.
-  const int ngx = (g.nx + XR - 1) / XR;
-  for (int t = threadIdx.x; t < ngx * nyz; t += T) {
-    const int grp = t / nyz, yz = t - grp * nyz;
+constexpr int XR = 4;  // outputs per thread of an axis stage: each load of the plane serves XR products
+
+// One stage of the DFT along an axis of n points at stride s (the plane is [outer][n][s]), then a barrier.
+// With n = n1 n2, x = n2 x1 + x2 and k = k1 + n1 k2,
+//   FIRST:  out[n1 x2 + k1] = sum_x1 in[n2 x1 + x2] w^{k1 (n2 x1 + x2)}   (terms = n1; the twiddle between the stages rides
+//                                                                          along in the exponent)
+//   else:   out[k1 + n1 k2] = sum_x2 in[n1 x2 + k1] w^{n1 x2 k2}          (terms = n2)
+// Neighbouring threads take neighbouring elements of the stride s, then of x2 (FIRST) or k1: the plane's loads are
+// conflict-free and the twiddles mostly broadcast.
+template <bool FIRST>
+__device__ __forceinline__ void dft_axis_stage(const double2* in, double2* out, const double2* tw, int n, int n1, int n2,
+                                               int s, int nk) {
+  const int terms = FIRST ? n1 : n2, other = FIRST ? n2 : n1;
+  const int rest = nk / terms, groups = (terms + XR - 1) / XR;
+  const int step_in = (FIRST ? n2 : n1) * s;
+  for (int t = threadIdx.x; t < groups * rest; t += blockDim.x) {
+    const int grp = t / rest, r = t - grp * rest;
+    const int i = r % s, q = r / s, j = q % other, o = q / other;  // j: x2 (FIRST) or k1
+    const double2* p = in + (size_t)o * n * s + j * s + i;
     double2 acc[XR];
-    int m[XR], kx[XR];
+    int m[XR], dm[XR];
 #pragma unroll
-    for (int j = 0; j < XR; ++j) {
-      acc[j] = make_double2(0.0, 0.0);
-      m[j] = 0;
-      kx[j] = min(grp + j * ngx, g.nx - 1);  // outputs past nx are computed on a valid index and dropped
+    for (int u = 0; u < XR; ++u) {
+      const int k = min(grp + u * groups, terms - 1);  // outputs past the end are computed on a valid index and dropped
+      acc[u] = make_double2(0.0, 0.0);
+      m[u] = FIRST ? k * j : 0;  // k j < n1 n2, and k n2 or k n1 < n
+      dm[u] = FIRST ? k * n2 : k * n1;
     }
-    for (int x = 0; x < g.nx; ++x) {
-      const double2 v = in[x * nyz + yz];
+    for (int x = 0; x < terms; ++x) {
+      const double2 v = p[x * step_in];
 #pragma unroll
-      for (int j = 0; j < XR; ++j) {
-        cfma(acc[j], v, twx[m[j]]);
-        m[j] += kx[j];
-        if (m[j] >= g.nx) m[j] -= g.nx;
+      for (int u = 0; u < XR; ++u) {
+        cfma(acc[u], v, tw[m[u]]);
+        m[u] += dm[u];
+        if (m[u] >= n) m[u] -= n;
       }
     }
+    double2* d = out + (size_t)o * n * s + i;
 #pragma unroll
-    for (int j = 0; j < XR; ++j)
-      if (grp + j * ngx < g.nx) out[(grp + j * ngx) * nyz + yz] = acc[j];
+    for (int u = 0; u < XR; ++u) {
+      const int k = grp + u * groups;
+      if (k < terms) d[(FIRST ? n1 * j + k : j + n1 * k) * s] = acc[u];
+    }
   }
   __syncthreads();
 }
 
-// out[kx][y][z] = sum_x in[x][y][z] * twx[(kx*x) % nx], then along y, then z (skipped when the axis has
-// length 1).  Result ends in `a` (the input buffer); `b` is work space.  Both buffers hold g.nk points.
-__device__ void plane_dft(double2* a, double2* b, const double2* s_tw, const Grid3 g) {
-  const int T = blockDim.x;
-  const double2* twx = s_tw;
-  const double2* twy = s_tw + g.nx;
-  const double2* twz = s_tw + g.nx + g.ny;
-  const int nyz = g.ny * g.nz;
-  dft_axis_x(a, b, twx, g);  // x axis: a -> b
-  const int ngx = (g.nx + XR - 1) / XR;
-  // y axis: b -> a.  A thread computes the outputs of one (ky, z) for the rows kx = grp + j ngx (j < XR), so each
-  // twiddle load (distinct across the lanes) serves XR products and the row loads are warp broadcasts; every
-  // output still sums over y in order.
-  for (int t = threadIdx.x; t < ngx * nyz; t += T) {
-    const int grp = t / nyz, r = t - grp * nyz;
-    const int ky = r / g.nz, z = r - ky * g.nz;
-    double2 acc[XR];
-    const double2* row[XR];
-#pragma unroll
-    for (int j = 0; j < XR; ++j) {
-      acc[j] = make_double2(0.0, 0.0);
-      row[j] = b + min(grp + j * ngx, g.nx - 1) * nyz + z;  // rows past nx are read on a valid row and dropped
-    }
-    int m = 0;
-    for (int y = 0; y < g.ny; ++y) {
-      const double2 w = twy[m];
-#pragma unroll
-      for (int j = 0; j < XR; ++j) cfma(acc[j], row[j][y * g.nz], w);
-      m += ky;
-      if (m >= g.ny) m -= g.ny;
-    }
-#pragma unroll
-    for (int j = 0; j < XR; ++j)
-      if (grp + j * ngx < g.nx) a[(grp + j * ngx) * nyz + r] = acc[j];
+// One axis of the plane in a; on return a is the buffer that holds the result.
+__device__ __forceinline__ void dft_axis(double2*& a, double2*& b, const double2* tw, int n, int n1, int s, int nk) {
+  if (n == 1) return;
+  if (n1 > 1) {
+    dft_axis_stage<true>(a, b, tw, n, n1, n / n1, s, nk);
+    dft_axis_stage<false>(b, a, tw, n, n1, n / n1, s, nk);
+  } else {
+    dft_axis_stage<false>(a, b, tw, n, 1, n, s, nk);
+    double2* t = a;
+    a = b;
+    b = t;
   }
-  __syncthreads();
-  if (g.nz > 1) {
-    for (int e = threadIdx.x; e < g.nk; e += T) {
-      const int base = (e / g.nz) * g.nz, kz = e - base;
-      double2 acc = make_double2(0.0, 0.0);
-      int m = 0;
-      for (int z = 0; z < g.nz; ++z) {
-        cfma(acc, a[base + z], twz[m]);
-        m += kz;
-        if (m >= g.nz) m -= g.nz;
-      }
-      b[e] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < g.nk; e += T) a[e] = b[e];
-    __syncthreads();
-  }
+}
+
+// out[kx][ky][kz] = sum_xyz in[x][y][z] twx[kx x % nx] twy[ky y % ny] twz[kz z % nz], axis by axis, of the
+// plane in a with b as work space (g.nk points each).  Returns the one of the two that holds the result.
+__device__ double2* plane_dft(double2* a, double2* b, const double2* s_tw, const Grid3 g) {
+  dft_axis(a, b, s_tw, g.nx, g.fx, g.ny * g.nz, g.nk);
+  dft_axis(a, b, s_tw + g.nx, g.ny, g.fy, g.nz, g.nk);
+  dft_axis(a, b, s_tw + g.nx + g.ny, g.nz, g.fz, 1, g.nk);
+  return a;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -130,7 +128,11 @@ struct PlaneAddr {
   }
 };
 
-__global__ void __launch_bounds__(BZ_THREADS) dft_planes_kernel(const double2* __restrict__ in, PlaneAddr ia,
+// Threads of a plane's CTA: its strided loads and stores (16 bytes a sector, the planes being interleaved) are latency, so
+// larger planes get more threads.
+static inline int plane_threads(int nk) { return nk >= 1024 ? 512 : BZ_THREADS; }
+
+__global__ void __launch_bounds__(512) dft_planes_kernel(const double2* __restrict__ in, PlaneAddr ia,
                                                                  double2* __restrict__ out, PlaneAddr oa,
                                                                  int n_planes, Grid3 g,
                                                                  const double2* __restrict__ tw, double scale,
@@ -142,11 +144,12 @@ __global__ void __launch_bounds__(BZ_THREADS) dft_planes_kernel(const double2* _
   load_twiddles(s_tw, tw, g);
   for (int p = blockIdx.x; p < n_planes; p += gridDim.x) {
     __syncthreads();
+#pragma unroll 8
     for (int r = threadIdx.x; r < g.nk; r += blockDim.x) a[r] = in[ia.at(p, gather ? gather[r] : r)];
     __syncthreads();
-    plane_dft(a, b, s_tw, g);
+    const double2* res = plane_dft(a, b, s_tw, g);
     for (int r = threadIdx.x; r < g.nk; r += blockDim.x) {
-      double2 v = a[r];
+      double2 v = res[r];
       out[oa.at(p, r)] = make_double2(v.x * scale, v.y * scale);
     }
   }
@@ -587,12 +590,12 @@ __global__ void __launch_bounds__(BZ_THREADS, MAXR <= 4 ? 3 : 1) sigma_partial_k
           Pa[r] = kv;
         }
         __syncthreads();
-        plane_dft(Pa, Pb, s_tw, g);
+        const double2* kr = plane_dft(Pa, Pb, s_tw, g);
         const double2* gp = g_r + (((size_t)(v - w + niw) * nb + a) * nb + d) * g.nk;
 #pragma unroll
         for (int k = 0; k < MAXR; ++k) {
           const int r = threadIdx.x + k * BZ_THREADS;
-          if (r < g.nk) cfma(acc[k], gp[r], Pa[r]);
+          if (r < g.nk) cfma(acc[k], gp[r], kr[r]);
         }
       }
     }
@@ -683,11 +686,11 @@ int dga_dft_planes_c128(const void* in, long long in_s_hi, long long in_s_lo, lo
     dga_set_error("dga_dft_planes_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   PlaneAddr ia{in_s_hi, in_s_lo, in_s_r, n_lo}, oa{out_s_hi, out_s_lo, out_s_r, n_lo};
   const size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
   cudaFuncSetAttribute(dft_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dft_planes_kernel<<<grid_cap(n_planes), BZ_THREADS, smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
+  dft_planes_kernel<<<grid_cap(n_planes), plane_threads(g.nk), smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
                                                                       n_planes, g, (const double2*)tw, scale, nullptr);
   return launch_status("dga_dft_planes_c128");
 }
@@ -703,11 +706,11 @@ int dga_dft_planes_gather_c128(const void* in, long long in_s_hi, long long in_s
     dga_set_error("dga_dft_planes_gather_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   PlaneAddr ia{in_s_hi, in_s_lo, in_s_r, n_lo}, oa{out_s_hi, out_s_lo, out_s_r, n_lo};
   const size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
   cudaFuncSetAttribute(dft_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dft_planes_kernel<<<grid_cap(n_planes), BZ_THREADS, smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
+  dft_planes_kernel<<<grid_cap(n_planes), plane_threads(g.nk), smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
                                                                       n_planes, g, (const double2*)tw, scale, gather);
   return launch_status("dga_dft_planes_gather_c128");
 }
@@ -723,7 +726,7 @@ int dga_bubble_c128(const void* g_r, int n_orb, int niv, int niw, int nx, int ny
     dga_set_error("dga_bubble_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   OutStrides7 os{out_strides[0], out_strides[1], out_strides[2], out_strides[3],
                  out_strides[4], out_strides[5], out_strides[6]};
   if ((long long)n_qirr > (long long)g.nk) {
@@ -760,7 +763,7 @@ int dga_sigma_wedge_c128(const void* kern, const void* g_r, int n_orb, int niv, 
     dga_set_error("dga_sigma_wedge_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   const int n2 = n_orb * n_orb;
   const size_t need = dga_sigma_wedge_scratch_bytes(n_orb, niv, niw, n_q, g.nk, n_chunks);
   if (scratch_bytes < need) {
@@ -797,7 +800,7 @@ int dga_sigma_wedge_c128(const void* kern, const void* g_r, int n_orb, int niv, 
   const size_t dsmem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
   cudaFuncSetAttribute(dft_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsmem);
   PlaneAddr pa{(long long)g.nk, 0, 1, 1};
-  dft_planes_kernel<<<grid_cap(niv * n2), BZ_THREADS, dsmem, stream>>>(sig, pa, part, pa, niv * n2, g,
+  dft_planes_kernel<<<grid_cap(niv * n2), plane_threads(g.nk), dsmem, stream>>>(sig, pa, part, pa, niv * n2, g,
                                                                        (const double2*)tw_inv, 1.0 / (double)g.nk,
                                                                        nullptr);
   if (launch_status("dga_sigma_wedge_c128")) return DGA_ERR_LAUNCH;
@@ -885,7 +888,7 @@ int dga_sigma_rspace_c128(const void* kern, const void* g_r, int n_orb, int niv,
     dga_set_error("dga_sigma_rspace_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   const size_t need = dga_sigma_scratch_bytes(n_orb, niv, g.nk, n_chunks);
   if (scratch_bytes < need) {
     dga_set_error("dga_sigma_rspace_c128: scratch too small (%zu < %zu)", scratch_bytes, need);
@@ -911,7 +914,7 @@ int dga_sigma_c128(const void* kern, const void* g_r, int n_orb, int niv, int ni
     dga_set_error("dga_sigma_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  Grid3 g{nx, ny, nz, nx * ny * nz};
+  const Grid3 g = make_grid(nx, ny, nz);
   const int n2 = n_orb * n_orb;
   const size_t need = dga_sigma_scratch_bytes(n_orb, niv, g.nk, n_chunks);
   if (scratch_bytes < need) {
@@ -927,7 +930,7 @@ int dga_sigma_c128(const void* kern, const void* g_r, int n_orb, int niv, int ni
   size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
   cudaFuncSetAttribute(dft_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   PlaneAddr pa{(long long)g.nk, 0, 1, 1};
-  dft_planes_kernel<<<grid_cap(niv * n2), BZ_THREADS, smem, stream>>>(sig, pa, part, pa, niv * n2, g,
+  dft_planes_kernel<<<grid_cap(niv * n2), plane_threads(g.nk), smem, stream>>>(sig, pa, part, pa, niv * n2, g,
                                                                       (const double2*)tw_inv, 1.0 / (double)g.nk,
                                                                       nullptr);
   if (launch_status("dga_sigma_c128")) return DGA_ERR_LAUNCH;
