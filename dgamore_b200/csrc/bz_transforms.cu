@@ -737,7 +737,12 @@ int dga_bubble_c128(const void* g_r, int n_orb, int niv, int niw, int nx, int ny
                       (6 * (size_t)n_qirr + 1) * sizeof(int);
   cudaFuncSetAttribute(bubble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const long long work = (long long)(niw + 1) * 2 * niv * n_orb * n_orb;
-  const long long cap = 64LL * device_sm_count();
+  // Four CTAs per resident one: each numbers the (qy, qz) pairs of the q list once, a serial pass that takes longer than a
+  // plane at the larger grids (2.95 ms for 561 q of 64 x 64 when every plane's CTA repeated it, 1.44 ms now), and the last
+  // wave stays short.
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bubble_kernel, BZ_THREADS, smem);
+  const long long cap = 4LL * (per_sm > 0 ? per_sm : 1) * device_sm_count();
   bubble_kernel<<<(int)(work < cap ? work : cap), BZ_THREADS, smem, stream>>>(
       (const double2*)g_r, n_orb, niv, niw, g, q_irr, n_qirr, (const double2*)tw, beta, (double2*)out, os);
   return launch_status("dga_bubble_c128");

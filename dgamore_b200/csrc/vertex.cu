@@ -13,6 +13,9 @@
 //   * dga_dc_kernel_c128:    K_dc = ((U_adcb / beta^2) chi0) . F_dc cut to the core box (nonlocal_sde.py:185-198),
 //                            a batched complex GEMM over w.
 #include "dga_common.cuh"
+#include "lu_dmma.cuh"
+
+#include <cooperative_groups.h>
 
 namespace dga {
 
@@ -233,19 +236,34 @@ __device__ double block_min(double v, double* red) {
   return r;
 }
 
-__global__ void lambda_kernel(const double2* __restrict__ chi, int Q, int W, const long long* __restrict__ weights,
-                              const double2* __restrict__ target, double beta, double nk_tot, double delta0,
-                              double eps, int maxiter, double* __restrict__ lambda_out, int* __restrict__ iters_out,
-                              int* __restrict__ status, double2* __restrict__ chi_out) {
-  __shared__ double red[32];
-  const int ch = blockIdx.x;
-  const double2* c = chi + (size_t)ch * Q * W;
-  const int niw = W - 1, nwf = 2 * niw + 1;
-  const long long total = (long long)Q * nwf;
+// One cluster of eight CTAs per channel.  1 / chi is taken once and kept in shared memory (LAMBDA_CACHED elements a CTA;
+// larger grids take it again per step), w < 0 is the conjugate of w > 0 (twice the real parts, the imaginary ones cancel),
+// and a step's four sums cross the cluster through distributed shared memory, in the same order on every CTA.  One CTA per
+// channel that formed every term from chi in each step took 70 us at 45 q x 41 frequencies and 660 us at 561 x 121;
+// this takes 33 and 96.
+constexpr int LAMBDA_CTAS = 8, LAMBDA_THREADS = 256, LAMBDA_CACHED = 8192;
+__global__ void __cluster_dims__(LAMBDA_CTAS, 1, 1) __launch_bounds__(LAMBDA_THREADS)
+    lambda_kernel(const double2* __restrict__ chi, int Q, int W, const long long* __restrict__ weights,
+                  const double2* __restrict__ target, double beta, double nk_tot, double delta0, double eps, int maxiter,
+                  double* __restrict__ lambda_out, int* __restrict__ iters_out, int* __restrict__ status,
+                  double2* __restrict__ chi_out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* inv_c = reinterpret_cast<double2*>(smem_raw);  // 1 / chi of this CTA's elements
+  __shared__ double red[LAMBDA_THREADS / 32][4];
+  __shared__ double part[2][4];  // this CTA's sums of a step, read by the cluster
+  __shared__ double scratch[32];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ch = blockIdx.x / LAMBDA_CTAS, tid = threadIdx.x;
+  const long long total = (long long)Q * W, per = (total + LAMBDA_CTAS - 1) / LAMBDA_CTAS;
+  const long long e0 = rank * per, e1 = min(total, e0 + per);
+  const int n = e1 > e0 ? (int)(e1 - e0) : 0, n_cached = min(n, LAMBDA_CACHED);
+  const double2* c = chi + (size_t)ch * total;
+  for (int i = tid; i < n_cached; i += LAMBDA_THREADS) inv_c[i] = crecip(c[e0 + i]);
   // lambda_start = -min_q 1 / Re chi(q, w = 0)
   double mn = INFINITY;
-  for (int q = threadIdx.x; q < Q; q += blockDim.x) mn = fmin(mn, 1.0 / c[(size_t)q * W].x);
-  const double lam0 = -block_min(mn, red);
+  for (int q = tid; q < Q; q += LAMBDA_THREADS) mn = fmin(mn, 1.0 / c[(size_t)q * W].x);
+  const double lam0 = -block_min(mn, scratch);
   const double factor = 1.0 / beta / nk_tot;
   const double2 tgt = target[ch];
   double delta = delta0;
@@ -253,30 +271,45 @@ __global__ void lambda_kernel(const double2* __restrict__ chi, int Q, int W, con
   double result = lam;
   int it = 0, converged = 0;
   for (; it < maxiter; ++it) {
-    double s1r = 0.0, s1i = 0.0, s2r = 0.0, s2i = 0.0;
-    for (long long e = threadIdx.x; e < total; e += blockDim.x) {
-      const int q = (int)(e / nwf);
-      const int wf = (int)(e - (long long)q * nwf);
-      const int w = wf - niw;
-      double2 x = c[(size_t)q * W + (w < 0 ? -w : w)];
-      if (w < 0) x.y = -x.y;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = tid; i < n; i += LAMBDA_THREADS) {
+      const long long e = e0 + i;
+      const int q = (int)(e / W), w = (int)(e - (long long)q * W);
       // chi_lam = 1 / (1 / chi + lam)
-      double2 inv = crecip(x);
+      double2 inv = i < n_cached ? inv_c[i] : crecip(c[e]);
       inv.x += lam;
-      const double2 cl = crecip(inv);
+      const double2 cl = crecip(inv), cl2 = cmul(cl, cl);
       const double wq = (double)weights[q];
-      s1r += wq * cl.x;
-      s1i += wq * cl.y;
-      const double2 cl2 = cmul(cl, cl);
-      s2r += wq * cl2.x;
-      s2i += wq * cl2.y;
+      const double wr = w ? 2.0 * wq : wq, wi = w ? 0.0 : wq;
+      s[0] += wr * cl.x;
+      s[1] += wi * cl.y;
+      s[2] += wr * cl2.x;
+      s[3] += wi * cl2.y;
     }
-    s1r = block_sum(s1r, red);
-    s1i = block_sum(s1i, red);
-    s2r = block_sum(s2r, red);
-    s2i = block_sum(s2i, red);
-    const double2 f = make_double2(s1r * factor - tgt.x, s1i * factor - tgt.y);
-    const double2 fp = make_double2(-s2r * factor, -s2i * factor);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+    if ((tid & 31) == 0)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) red[tid >> 5][k] = s[k];
+    __syncthreads();
+    double* mine = part[it & 1];
+    if (tid < 4) {
+      double v = 0.0;
+      for (int wp = 0; wp < LAMBDA_THREADS / 32; ++wp) v += red[wp][tid];
+      mine[tid] = v;
+    }
+    cluster.sync();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = 0.0;
+    for (int r = 0; r < LAMBDA_CTAS; ++r) {
+      const double* theirs = cluster.map_shared_rank(mine, r);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) s[k] += theirs[k];
+    }
+    const double2 f = make_double2(s[0] * factor - tgt.x, s[1] * factor - tgt.y);
+    const double2 fp = make_double2(-s[2] * factor, -s[3] * factor);
     const double lam_new = lam - cdiv(f, fp).x;
     if (fabs(f.x) < eps) {
       result = lam_new;
@@ -294,17 +327,18 @@ __global__ void lambda_kernel(const double2* __restrict__ chi, int Q, int W, con
     }
     result = lam;
   }
-  if (threadIdx.x == 0) {
+  if (rank == 0 && tid == 0) {
     lambda_out[ch] = result;
     if (iters_out) iters_out[ch] = it;
     if (status && !converged) atomicOr(status, DGA_ITEM_NOCONVERGE);
   }
   // apply to the half range
-  for (int e = threadIdx.x; e < Q * W; e += blockDim.x) {
-    double2 inv = crecip(c[e]);
+  for (int i = tid; i < n; i += LAMBDA_THREADS) {
+    double2 inv = i < n_cached ? inv_c[i] : crecip(c[e0 + i]);
     inv.x += result;
-    chi_out[(size_t)ch * Q * W + e] = crecip(inv);
+    chi_out[(size_t)ch * total + e0 + i] = crecip(inv);
   }
+  cluster.sync();  // no CTA leaves while another may read its sums
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -313,25 +347,28 @@ __global__ void lambda_kernel(const double2* __restrict__ chi, int Q, int W, con
 //   chi0_inv: [Q][W][nv][n2][n2]; X: [2][Q][W][N][n2]; uv: [2][Q][n2][n2]; chi_phys: [2][Q][W][n2][n2]
 //   k_dc: [Q][W][nv][n2][n2] or null;  out K: [Q][W][nv][n2][n2];  gamma_out (optional): [2][Q][W][nv][n2][n2]
 // ------------------------------------------------------------------------------------------------
-constexpr int KA_WARPS = 8;  // matrices per block
-// One warp per matrix (q, w, nu); the n2 x n2 products run with the orbital-pair count NN2 fixed at compile time
-// (elements per lane EPL), four blocks per SM (two for 4 orbitals, whose accumulators need the registers) to hide
-// the latency of the dependent product chain.
+constexpr int KA_WARPS = 8;
+// Lanes per matrix (q, w, nu): a matrix of one or 16 elements shares its warp with others (one warp per element left 31 of
+// 32 lanes idle with one orbital: 2.0 ms for 561 x 61 x 120 matrices, 0.08 now; 0.95 and 0.80 ms with two orbitals, 325 x
+// 31 x 60).
+__host__ __device__ constexpr int ka_lanes(int n2) { return n2 == 1 ? 1 : n2 == 4 ? 16 : 32; }
+// The n2 x n2 products run with the orbital-pair count NN2 fixed at compile time (elements per lane EPL), four blocks per SM
+// (two for 4 orbitals, whose accumulators need the registers) to hide the latency of the dependent product chain.
 template <int NN2>
 __global__ void __launch_bounds__(32 * KA_WARPS, NN2 > 9 ? 2 : 4)
 kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __restrict__ X,
                                        const double2* __restrict__ uv, const double2* __restrict__ chi_phys,
                                        const double2* __restrict__ k_dc, int nv, int W, int Q, double beta,
                                        double2* __restrict__ K, double2* __restrict__ gamma_out) {
-  constexpr int n2 = NN2, nn = NN2 * NN2, EPL = (nn + 31) / 32;
+  constexpr int n2 = NN2, nn = NN2 * NN2, GL = ka_lanes(NN2), EPL = (nn + GL - 1) / GL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double2* g3 = reinterpret_cast<double2*>(smem_raw) + (size_t)wib * 3 * nn;
+  const int lane = threadIdx.x % GL, slot = threadIdx.x / GL;
+  double2* g3 = reinterpret_cast<double2*>(smem_raw) + (size_t)slot * 3 * nn;
   double2* t1 = g3 + nn;
   double2* t2 = t1 + nn;
-  const long long t = blockIdx.x * (long long)KA_WARPS + wib;
-  const long long total = (long long)Q * W * nv;
-  if (t >= total) return;  // the whole warp; the block has no block-wide barrier
+  const long long total = (long long)Q * W * nv, mine = blockIdx.x * (long long)(32 * KA_WARPS / GL) + slot;
+  const bool valid = mine < total;  // the others of the warp's matrices go on: its barriers are the warp's
+  const long long t = valid ? mine : total - 1;
   const int v = (int)(t % nv);
   const long long qw = t / nv;
   const int q = (int)(qw / W);
@@ -340,7 +377,7 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
   double2 acc[EPL];
 #pragma unroll
   for (int j = 0; j < EPL; ++j) {
-    const int e = lane + 32 * j;
+    const int e = lane + GL * j;
     acc[j] = make_double2(0.0, 0.0);
     if (e < nn && k_dc) {
       const double2 z = k_dc[(size_t)t * nn + e];
@@ -356,7 +393,7 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
     // gamma = beta * (chi0_inv @ X_nu)
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
-      const int e = lane + 32 * j;
+      const int e = lane + GL * j;
       if (e < nn) {
         const int p = e / n2, sidx = e - p * n2;
         double2 a = make_double2(0.0, 0.0);
@@ -364,13 +401,13 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
         for (int m = 0; m < n2; ++m) cfma(a, c0i[p * n2 + m], x[(size_t)(m * nv + v) * n2 + sidx]);
         const double2 g = make_double2(beta * a.x, beta * a.y);
         g3[e] = g;
-        if (go) go[e] = g;
+        if (go && valid) go[e] = g;
       }
     }
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {  // t1 = gamma @ U_r
-      const int e = lane + 32 * j;
+      const int e = lane + GL * j;
       if (e < nn) {
         const int p = e / n2, sidx = e - p * n2;
         double2 a = make_double2(0.0, 0.0);
@@ -382,7 +419,7 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {  // t2 = gamma - t1 @ chi_r  (- 2/3 on the diagonal in the magnetic channel)
-      const int e = lane + 32 * j;
+      const int e = lane + GL * j;
       if (e < nn) {
         const int p = e / n2, sidx = e - p * n2;
         double2 a = make_double2(0.0, 0.0);
@@ -397,7 +434,7 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
     const double f = ch == 0 ? 1.0 : 3.0;
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {  // K += f U_r @ t2
-      const int e = lane + 32 * j;
+      const int e = lane + GL * j;
       if (e < nn) {
         const int p = e / n2, sidx = e - p * n2;
         double2 a = make_double2(0.0, 0.0);
@@ -412,8 +449,8 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
   double2* o = K + (size_t)t * nn;
 #pragma unroll
   for (int j = 0; j < EPL; ++j) {
-    const int e = lane + 32 * j;
-    if (e < nn) o[e] = acc[j];
+    const int e = lane + GL * j;
+    if (e < nn && valid) o[e] = acc[j];
   }
 }
 
@@ -421,21 +458,33 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
 // K1 = (U_adcb / beta^2) @ chi0 for every (q, w, nu_full): one warp per matrix, written as the row-major GEMM
 // operand K1[w][(q, p)][(m, nu)] (row (q, p), column (m, nu), Kd = n2 * nvf columns)
 // ------------------------------------------------------------------------------------------------
-__global__ void dc_left_kernel(const double2* __restrict__ chi0, const double2* __restrict__ u_perm, int n2, int Q,
-                               int W, int nvf, double2* __restrict__ k1) {
-  // one warp per matrix t = (q, w, nu), lane l computing the elements l, l + 32, ...
-  const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= (long long)Q * W * nvf) return;
-  const int nu = (int)(t % nvf), qw = (int)(t / nvf), w = qw % W, q = qw / W;
-  const int nn = n2 * n2, Kd = n2 * nvf;
-  const double2* c = chi0 + (size_t)t * nn;
-  double2* o = k1 + ((size_t)w * Q + q) * n2 * Kd + nu;
-  for (int e = lane; e < nn; e += 32) {
-    const int i = e / n2, j = e - i * n2;
+// A CTA takes DL_MATS / n2^2 (at least 16) frequencies of one (q, w): the matrices come in as they lie, and the products
+// leave with nu fastest, as k1 holds them. (One warp per matrix wrote 16 bytes at a time, and with one orbital used one
+// lane: 0.94 ms for 561 x 61 x 120 of them, 0.08 now; 0.77 and 0.47 ms for 153 x 41 x 80 of three orbitals.)
+constexpr int DL_MATS = 1024;
+__host__ __device__ inline int dc_left_nus(int n2, int nvf) {
+  const int nus = DL_MATS / (n2 * n2) > 16 ? DL_MATS / (n2 * n2) : 16;
+  return nus < nvf ? nus : nvf;
+}
+__global__ void __launch_bounds__(256) dc_left_kernel(const double2* __restrict__ chi0,
+                                                      const double2* __restrict__ u_perm, int n2, int Q, int W, int nvf,
+                                                      int nus, double2* __restrict__ k1) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* c = reinterpret_cast<double2*>(smem_raw);  // [nus][nn | 1]: odd pitch, so that lanes along nu hit all banks
+  const int nn = n2 * n2, ld = nn | 1, Kd = n2 * nvf;
+  const int chunks = (nvf + nus - 1) / nus;
+  const long long qw = blockIdx.x / chunks;
+  const int nu0 = (int)(blockIdx.x % chunks) * nus, cnt = min(nus, nvf - nu0);
+  const int w = (int)(qw % W), q = (int)(qw / W);
+  const double2* src = chi0 + ((size_t)qw * nvf + nu0) * nn;
+  for (int e = threadIdx.x; e < cnt * nn; e += blockDim.x) c[(e / nn) * ld + e % nn] = src[e];
+  __syncthreads();
+  double2* o = k1 + ((size_t)w * Q + q) * n2 * Kd + nu0;
+  for (int e = threadIdx.x; e < cnt * nn; e += blockDim.x) {
+    const int nu = e % cnt, ij = e / cnt, i = ij / n2, j = ij - i * n2;
     double2 a = make_double2(0.0, 0.0);
-    for (int k = 0; k < n2; ++k) cfma(a, u_perm[i * n2 + k], c[k * n2 + j]);
-    o[(size_t)i * Kd + (size_t)j * nvf] = a;
+    for (int k = 0; k < n2; ++k) cfma(a, u_perm[i * n2 + k], c[nu * ld + k * n2 + j]);
+    o[(size_t)i * Kd + (size_t)j * nvf + nu] = a;
   }
 }
 
@@ -453,13 +502,16 @@ struct DcGemmArgs {
 
 constexpr int DG_TM = 64, DG_TN = 64, DG_TK = 16;
 
+// 64 x 64 output tile per CTA on the FP64 tensor pipe, 16 x 32 per warp; the pitch DG_T? + 2 spreads a fragment's four k
+// over the banks. 41 products of 1,377 x 720 x 720 take 7.8 ms (30 TFLOP/s), 10.9 as 4 x 4 vector-pipe tiles.
 __global__ void __launch_bounds__(256, 2) dc_gemm_kernel(DcGemmArgs a) {
-  __shared__ double2 As[DG_TK][DG_TM + 1];
-  __shared__ double2 Bs[DG_TK][DG_TN];
+  __shared__ double2 As[DG_TK][DG_TM + 2];
+  __shared__ double2 Bs[DG_TK][DG_TN + 2];
   const int w = blockIdx.z;
   const int M = a.Q * a.n2, Kd = a.n2 * a.nvf, Nc = a.n2 * a.nv;
   const int r0 = blockIdx.y * DG_TM, c0 = blockIdx.x * DG_TN;
-  const int tid = threadIdx.x, ty = tid & 15, tx = tid >> 4;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wr = (tid >> 5) % 4 * 16, wc = (tid >> 5) / 4 * 32;  // this warp's part of the tile
   const int Nf = a.n2 * a.nvf;
   const double2* A = a.k1 + (size_t)w * M * Kd;
   const double2* B = a.fdc + (size_t)w * Nf * Nf;
@@ -481,11 +533,11 @@ __global__ void __launch_bounds__(256, 2) dc_gemm_kernel(DcGemmArgs a) {
       rb_v[i] = (bcol >= 0 && kr < Kd) ? B[(size_t)kr * Nf + bcol] : make_double2(0.0, 0.0);
     }
   };
-  double2 acc[4][4];
+  CAcc acc[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int n = 0; n < 4; ++n)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0.0, 0.0);
+    for (int i = 0; i < 4; ++i) acc[n].re[i] = acc[n].im[i] = 0.0;
   load(0);
   for (int k0 = 0; k0 < Kd; k0 += DG_TK) {
 #pragma unroll
@@ -496,30 +548,26 @@ __global__ void __launch_bounds__(256, 2) dc_gemm_kernel(DcGemmArgs a) {
     __syncthreads();
     if (k0 + DG_TK < Kd) load(k0 + DG_TK);
 #pragma unroll
-    for (int kk = 0; kk < DG_TK; ++kk) {
-      double2 av[4], bv[4];
+    for (int kk = 0; kk < DG_TK; kk += 4) {
+      double2 b[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) cfma(acc[i][j], av[i], bv[j]);
+      for (int n = 0; n < 4; ++n) b[n] = Bs[kk + t][wc + n * 8 + g];
+      cdmma_row<4>(acc, As[kk + t][wr + g], As[kk + t][wr + g + 8], b);
     }
     __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = r0 + ty + 16 * i;
+    const int row = r0 + wr + g + (i < 2 ? 0 : 8);
     if (row >= M) continue;
     const int q = row / a.n2, p = row - q * a.n2;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = c0 + tx + 16 * j;
+    for (int n = 0; n < 4; ++n) {
+      const int col = c0 + wc + n * 8 + 2 * t + (i & 1);
       if (col >= Nc) continue;
       const int sidx = col / a.nv, nup = col - sidx * a.nv;
-      a.out[((((size_t)q * a.W + w) * a.nv + nup) * a.n2 + p) * a.n2 + sidx] = acc[i][j];
+      a.out[((((size_t)q * a.W + w) * a.nv + nup) * a.n2 + p) * a.n2 + sidx] =
+          make_double2(acc[n].re[i], acc[n].im[i]);
     }
   }
 }
@@ -597,9 +645,13 @@ int dga_lambda_c128(const void* chi, int n_q, int niw_half, int n_ch, const long
     dga_set_error("dga_lambda_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  lambda_kernel<<<n_ch, 1024, 0, stream>>>((const double2*)chi, n_q, niw_half, weights, (const double2*)target, beta,
-                                           nk_tot, delta, eps, maxiter, lambda_out, iters_out, status,
-                                           (double2*)chi_out);
+  const long long per = ((long long)n_q * niw_half + LAMBDA_CTAS - 1) / LAMBDA_CTAS;
+  const size_t smem = (size_t)(per < LAMBDA_CACHED ? per : LAMBDA_CACHED) * sizeof(double2);
+  cudaFuncSetAttribute(lambda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  lambda_kernel<<<n_ch * LAMBDA_CTAS, LAMBDA_THREADS, smem, stream>>>((const double2*)chi, n_q, niw_half, weights,
+                                                                      (const double2*)target, beta, nk_tot, delta, eps,
+                                                                      maxiter, lambda_out, iters_out, status,
+                                                                      (double2*)chi_out);
   return vstatus("dga_lambda_c128");
 }
 
@@ -612,8 +664,9 @@ int dga_kernel_assembly_c128(const void* chi0_inv, const void* X, const void* uv
     return DGA_ERR_ARG;
   }
   const long long total = (long long)n_q * niw_half * 2 * niv_core;
-  const size_t smem = (size_t)KA_WARPS * 3 * n2 * n2 * sizeof(double2);
-  const int blocks = (int)((total + KA_WARPS - 1) / KA_WARPS);
+  const int per_block = 32 * KA_WARPS / ka_lanes(n2);
+  const size_t smem = (size_t)per_block * 3 * n2 * n2 * sizeof(double2);
+  const int blocks = (int)((total + per_block - 1) / per_block);
 #define DGA_KA_CASE(NN)                                                                                        \
   case NN:                                                                                                     \
     cudaFuncSetAttribute(kernel_assembly_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
@@ -652,9 +705,16 @@ int dga_dc_kernel_c128(const void* chi0, const void* u_perm, const void* fdc, in
     dga_set_error("dga_dc_kernel_c128: scratch too small");
     return DGA_ERR_SCRATCH;
   }
-  const long long n_mats = (long long)n_q * niw_half * nvf;
-  dc_left_kernel<<<(int)((n_mats * 32 + 255) / 256), 256, 0, stream>>>((const double2*)chi0, (const double2*)u_perm, n2,
-                                                                  n_q, niw_half, nvf, (double2*)scratch);
+  const int nus = dc_left_nus(n2, nvf);
+  const long long left_blocks = (long long)n_q * niw_half * ((nvf + nus - 1) / nus);
+  if (left_blocks > 0x7fffffffLL) {
+    dga_set_error("dga_dc_kernel_c128: too many matrices");
+    return DGA_ERR_ARG;
+  }
+  const size_t left_smem = (size_t)nus * ((n2 * n2) | 1) * sizeof(double2);
+  cudaFuncSetAttribute(dc_left_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)left_smem);
+  dc_left_kernel<<<(int)left_blocks, 256, left_smem, stream>>>(
+      (const double2*)chi0, (const double2*)u_perm, n2, n_q, niw_half, nvf, nus, (double2*)scratch);
   if (vstatus("dga_dc_kernel_c128")) return DGA_ERR_LAUNCH;
   DcGemmArgs a;
   a.k1 = (const double2*)scratch;
