@@ -143,11 +143,10 @@ __global__ void eli_ladder_term_kernel(const double2* __restrict__ uv, const dou
   }
 }
 
-// Threads of an FP64 CTA: one warp up to N = 64 (29,600 factorisations of N = 40: 1.71 ms, 1.89 with two warps), two up to
-// N = 192 (14,208 of N = 120: 7.6 ms, 8.2 with one and 7.9 with four), four up to N = 512 (1,184 of N = 480: 18.2 ms, 18.6
-// with eight), eight above (592 of N = 720: 27.7 ms, 27.3 with four, whose panels hold eight rows a thread). Where the
-// items would fill less than half of the SMs' threads that way, each gets more: up to two rows a thread (441 items of
-// N = 200: 1.8 ms with four warps, 2.5 with two).
+// Threads of an FP64 CTA: one warp up to N = 64 (29,600 factorisations of N = 40: 1.45 ms, 1.79 with two warps), two up to
+// N = 192 (14,208 of N = 120: 6.8 ms, 7.6 with four), four up to N = 512 (1,184 of N = 480: 18.4 ms, 19.6 with eight), eight
+// above (592 of N = 720: 27.9 ms). Where the items would fill less than half of the SMs' threads that way, each gets more,
+// up to two rows a thread (441 items of N = 200: 1.8 ms with four warps, 2.5 with two).
 static int fp64_threads(int N, int n_items) {
   int nt = N <= 64 ? 32 : N <= LU_SMALL_N ? 64 : N <= 512 ? 128 : 256;
   while (nt < 256 && nt < N && (long)n_items * nt <= (long)device_sm_count() * 256) nt *= 2;

@@ -14,11 +14,8 @@
 // interleaved complex matrix are one 16-byte load per lane each (lane (g, t) holds row g and column t), so operands come
 // straight from L2 and L1: four warps per SM already reach 35 TFLOP/s. The tcgen05 pipe has no FP64 kind.
 //
-// What bounds it: the products at N = 720 (592 factorisations in 27.7 ms, 21.3 TFLOP/s, two CTAs an SM), waits on HBM and
-// L2 for the panels and the tiles' first elements below about N = 250 (14,208 of N = 120 in 7.6 ms, 8.7 TFLOP/s, 45% of the
-// warps' stalls). Whole passes, from the right-looking vector-pipe form to this one: 1,130 to 742 ms for three orbitals on
-// 32 x 32 (N = 720), 103 to 66 ms for one orbital on 64 x 64 (N = 120), 0.84 to 0.41 ms on 16 x 16 (N = 40), 404 to 165 ms
-// for the bilayer on 48 x 48 with its pairing box (N = 240, 124 right-hand sides).
+// What bounds it: the products at N = 720 (592 factorisations in 27.9 ms, 21.1 TFLOP/s, two CTAs an SM), waits on HBM and
+// L2 for the panels and the tiles' first elements below about N = 250 (14,208 of N = 120 in 6.8 ms, 9.6 TFLOP/s).
 #pragma once
 
 #include "dga_common.cuh"
@@ -32,17 +29,21 @@ constexpr int LU_RING = 4;  // steps of four columns a lane has in flight
 // Block width by the matrix size alone, so that a matrix goes through the same operations whatever CTA it is given. 16 up
 // to N = 192, where one or two warps take a matrix and 16 or 8 matrices share an SM (the shared memory of a 32-wide block
 // would admit five): the panels' chains of dependent steps, not the products, are what the time goes to. 29,600
-// factorisations of N = 40 took 1.71 ms against 2.90 at 32 wide, 9,472 of N = 160 8.7 against 9.2, each with its best
-// thread count; with many right-hand sides the wider block is the faster one from N = 240 (154 against 162 ms for the
+// factorisations of N = 40 take 1.45 ms, 2.79 in CTAs of 128 threads and 3.01 at 32 wide too; 9,472 of N = 160 8.2 against
+// 9.2; with many right-hand sides the wider block is the faster one from N = 240 (154 against 162 ms for the
 // bilayer pass with its pairing box).
 constexpr int LU_SMALL_N = 192;
 
-// Rows a thread holds in the panel and panel columns it keeps in registers, for matrices of up to RPT * NT rows: at most
-// RPT * PW = 16 complex values (64 registers).
+// Panel columns a thread can keep in registers with RPT rows (at most 16 complex values, 64 registers), and the columns
+// that are factored at a time: by the matrix size and the rows left alone, within what every thread count can keep there.
 template <int RPT>
 struct LuPanelWidth {
   static constexpr int value = RPT <= 2 ? 8 : RPT <= 4 ? 4 : 2;
 };
+__device__ __forceinline__ int lu_panel_width(int N, int m) {
+  const int rows = N <= LU_SMALL_N ? 64 : N <= 512 ? 128 : 256;  // the smallest thread count that takes N
+  return m <= 2 * rows ? 8 : m <= 4 * rows ? 4 : 2;
+}
 
 constexpr int LU_WARP_BUF = LU_RING * 2 * 33;
 
@@ -400,8 +401,9 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
   constexpr int PW = LuPanelWidth<RPT>::value, NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool singular = false;
-  for (int p0 = 0; p0 < nb; p0 += PW) {
-    const int pw = min(PW, nb - p0), jc = j0 + p0;
+  const int width = lu_panel_width(N, N - j0);  // <= PW
+  for (int p0 = 0; p0 < nb; p0 += width) {
+    const int pw = min(width, nb - p0), jc = j0 + p0;
     double2* P = A + (size_t)jc * ld;
     double2 a[RPT][PW];
     int pos[RPT];
@@ -544,29 +546,41 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
           }
       }
       __syncthreads();
+      // and applied to the rows below, 16 rows x 8 columns at a time on the tensor pipe (row by row on the vector pipe the
+      // update was a third of the panel: each of its many instructions waits behind the other matrices' products)
+      const int first = jc + pw, tiles = (N - first + 15) / 16, g = lane >> 2, t = lane & 3;
+      for (int tile = warp; tile < tiles; tile += NW) {
+        const int r0 = first + tile * 16 + g, r1 = r0 + 8;
+        const double2 *l0 = P + min(r0, N - 1), *l1 = P + min(r1, N - 1);
+        double2 x0[2], x1[2];
 #pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        if (pos[i] < jc + pw || pos[i] >= N) continue;
-        double2* row = P + (size_t)pw * ld + pos[i];
-        double2 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = u < rest ? row[(size_t)u * ld] : make_double2(0.0, 0.0);
+        for (int h = 0; h < 2; ++h) {
+          const bool in = h * 4 + t < pw;
+          x0[h] = in ? l0[(size_t)(h * 4 + t) * ld] : make_double2(0.0, 0.0);
+          x1[h] = in ? l1[(size_t)(h * 4 + t) * ld] : make_double2(0.0, 0.0);
+        }
 #pragma unroll 1
-        for (int c = 0; c < rest; c += 4) {  // four columns at a time, the next four on their way
-          double2 n[4];
+        for (int c0 = 0; c0 < rest; c0 += 8) {
+          double2 v[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            n[u] = c + 4 + u < rest ? row[(size_t)(c + 4 + u) * ld] : make_double2(0.0, 0.0);
+          for (int i = 0; i < 4; ++i) {
+            const int c = c0 + 2 * t + (i & 1), r = i < 2 ? r0 : r1;
+            v[i] = (c < rest && r < N) ? P[(size_t)(pw + c) * ld + r] : make_double2(0.0, 0.0);
+          }
+          CAcc acc[1];
 #pragma unroll
-          for (int k = 0; k < PW; ++k)
-            if (k < pw) {
+          for (int i = 0; i < 4; ++i) acc[0].re[i] = acc[0].im[i] = 0.0;
 #pragma unroll
-              for (int u = 0; u < 4; ++u) cfms(v[u], a[i][k], sm.us[k][c + u]);
+          for (int h = 0; h < 2; ++h)
+            if (h * 4 < pw) {
+              const double2 y[1] = {h * 4 + t < pw ? sm.us[h * 4 + t][c0 + g] : make_double2(0.0, 0.0)};
+              cdmma_row<1>(acc, x0[h], x1[h], y);
             }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (c + u < rest) row[(size_t)(c + u) * ld] = v[u];
-            v[u] = n[u];
+          for (int i = 0; i < 4; ++i) {
+            const int c = c0 + 2 * t + (i & 1), r = i < 2 ? r0 : r1;
+            if (c < rest && r < N)
+              P[(size_t)(pw + c) * ld + r] = make_double2(v[i].x - acc[0].re[i], v[i].y - acc[0].im[i]);
           }
         }
       }
