@@ -14,6 +14,7 @@
 // so the transform needs no plan and handles any grid: an axis of n = n1 n2 points, n1 the largest divisor up to sqrt(n),
 // takes n1 + n2 complex FMAs a point (14 instead of 48 at n = 48; a prime n is a direct sum).
 #include "dga_common.cuh"
+#include "lu_dmma.cuh"
 
 namespace dga {
 
@@ -314,19 +315,22 @@ __global__ void __launch_bounds__(BZ_THREADS, 3) bubble_kernel(const double2* __
 constexpr int SW_TK = 16;
 
 // C[p][r] = sum_q A[q][p] B[q][r]: A = K [Q][P] (planes contiguous), B = S [Q][Q], C = Kw [P][Q].  A TM x TN output
-// tile per 256-thread CTA, 4 x 4 per thread (TM * TN = 4096), K in steps of 16 with the next step's operands loaded
-// into registers while the current one multiplies.
+// tile per 256-thread CTA, 16 x 32 per warp on the FP64 tensor pipe (TM * TN = 4096), K in steps of 16 with the next step's
+// operands loaded into registers while the current one multiplies. 266k planes of 153 q take 1.95 ms (25 TFLOP/s), 2.77 as
+// 4 x 4 vector-pipe tiles; 7,320 of 561 q 0.74, 1.02 before.
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, 2) sigma_wedge_gemm_kernel(const double2* __restrict__ A,
                                                                   const double2* __restrict__ B, long long P, int Q,
                                                                   double2* __restrict__ C) {
-  static_assert(TM * TN == 4096, "4 x 4 outputs per thread of 256");
+  static_assert(TM * TN == 4096 && TN % 32 == 0, "16 x 32 outputs for each of eight warps");
   constexpr int AL = TM * SW_TK / 256, BL = TN * SW_TK / 256;  // tile elements loaded per thread
-  __shared__ double2 As[SW_TK][TM + 1];
-  __shared__ double2 Bs[SW_TK][TN];
+  // pitches that spread a fragment's four k over the banks
+  __shared__ double2 As[SW_TK][TM + 2];
+  __shared__ double2 Bs[SW_TK][TN + 2];
   const long long p0 = (long long)blockIdx.x * TM;
   const int r0 = blockIdx.y * TN;
-  const int tid = threadIdx.x, ty = tid % (TM / 4), tx = tid / (TM / 4);
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wr = (tid >> 5) % (TM / 16) * 16, wc = (tid >> 5) / (TM / 16) * 32;  // this warp's part of the tile
   double2 ra[AL], rb[BL];
   auto load = [&](int k0) {
 #pragma unroll
@@ -341,11 +345,11 @@ __global__ void __launch_bounds__(256, 2) sigma_wedge_gemm_kernel(const double2*
       rb[i] = (q < Q && r < Q) ? B[(size_t)q * Q + r] : make_double2(0.0, 0.0);
     }
   };
-  double2 acc[4][4];
+  CAcc acc[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int n = 0; n < 4; ++n)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_double2(0.0, 0.0);
+    for (int i = 0; i < 4; ++i) acc[n].re[i] = acc[n].im[i] = 0.0;
   load(0);
   for (int k0 = 0; k0 < Q; k0 += SW_TK) {
 #pragma unroll
@@ -361,27 +365,22 @@ __global__ void __launch_bounds__(256, 2) sigma_wedge_gemm_kernel(const double2*
     __syncthreads();
     if (k0 + SW_TK < Q) load(k0 + SW_TK);
 #pragma unroll
-    for (int kk = 0; kk < SW_TK; ++kk) {
-      double2 av[4], bv[4];
+    for (int kk = 0; kk < SW_TK; kk += 4) {
+      double2 b[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty + (TM / 4) * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + (TN / 4) * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) cfma(acc[i][j], av[i], bv[j]);
+      for (int n = 0; n < 4; ++n) b[n] = Bs[kk + t][wc + n * 8 + g];
+      cdmma_row<4>(acc, As[kk + t][wr + g], As[kk + t][wr + g + 8], b);
     }
     __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const long long p = p0 + ty + (TM / 4) * i;
+    const long long p = p0 + wr + g + (i < 2 ? 0 : 8);
     if (p >= P) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int r = r0 + tx + (TN / 4) * j;
-      if (r < Q) C[(size_t)p * Q + r] = acc[i][j];
+    for (int n = 0; n < 4; ++n) {
+      const int r = r0 + wc + n * 8 + 2 * t + (i & 1);
+      if (r < Q) C[(size_t)p * Q + r] = make_double2(acc[n].re[i], acc[n].im[i]);
     }
   }
 }
