@@ -295,7 +295,8 @@ def time_pass(lp, args, world: int, local: int, sample_clocks: bool):
 # single-wave launch of the same kernel on the 3-orbital case with the full N = 720 (4x4 grid, niw = 10,
 # 132 items); traffic grows in proportion to the items, so a full launch's traffic is items x this.
 DRAM_BYTES_PER_ITEM = {
-    "bse_solve_sum_fp64_kernel": 22.89e9 / 132,
+    # 8x8 grid, niw = 19: 600 items, about two waves (dram__bytes.sum.per_second x duration)
+    "bse_solve_sum_fp64_kernel": 73.67e9 / 600,
     "bse_panel_mixed_kernel": (5.670e9 + 4.917e9) / 132,
     "bse_panel_mixed_kernel<TC> (tcgen05 trailing tiles)": (6.093e9 + 4.978e9) / 132,
     "bse_solve_sum_mixed_kernel": 11.79e9 / 132,

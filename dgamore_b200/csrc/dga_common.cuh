@@ -38,9 +38,9 @@ typedef struct {
 
 // Launch choices of the BSE solvers (the search space of the autotuner); layout is part of the C ABI.
 typedef struct {
-  int kernel;       // 0 = default, 1 = shared-memory-panel kernel (mixed form only), 2 = 128-thread kernel,
+  int kernel;       // 0 = default, 1 = shared-memory-panel kernel (mixed form only), 2 = 128-thread (mixed) / FP64 kernel,
                     // 3 = shared-memory-panel kernel with tensor-core (tcgen05) trailing tiles (mixed form only)
-  int ctas_per_sm;  // CTAs per SM of the 128-thread kernels (0 = as many as fit)
+  int ctas_per_sm;  // CTAs per SM of kernel 2 (0 = as many as fit)
   long long wait_limit;  // polls of each bounded wait on a copy or tile inside an item (0 = the default limit)
 } dga_bse_tuning;
 

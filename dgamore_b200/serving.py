@@ -51,7 +51,7 @@ def _stream() -> ctypes.c_void_p:
 def launch_class(lp: LadderPass, precision: str) -> tuple:
     """Requests of one class share a batch launch: the same kernel as each would take alone
     (dga_bse_default_kernel), so that a request's results are bitwise the same in a batch and alone.  The
-    128-thread kernels and the mixed form's block kernel for 1 to 3 orbitals choose the right-hand-side count per
+    FP64 and 128-thread kernels and the mixed form's block kernel for 1 to 3 orbitals choose the right-hand-side count per
     item, so their requests share one launch whatever their orbital counts; the shared-memory-panel kernels and
     the 4-orbital block kernel are compiled per orbital count, so there the class also holds n_orb."""
     mixed = precision == "mixed"

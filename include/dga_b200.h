@@ -147,11 +147,12 @@ int dga_bse_resolve_fp64_c128(int n_orb, int niv, int niw_half, int n_q, int n_c
 
 /* Launch choices of the BSE solvers, the search space of the autotuner (dgamore_b200/autotune.py); no
  * counterpart in the upstream.  kernel: 0 = default (dga_bse_default_kernel), 1 = shared-memory-panel kernel
- * (mixed form only, N up to about 790), 2 = 128-thread kernel, 3 = shared-memory-panel kernel whose trailing
+ * (mixed form only, N up to about 790), 2 = 128-thread kernel (the only choice of the FP64 form, whose
+ * CTAs have 32 to 256 threads by size), 3 = shared-memory-panel kernel whose trailing
  * tiles run on the tensor cores (tcgen05.mma kind::tf32 with a three-term split for FP32-level products,
  * accumulators in tensor memory; mixed form only), 4 = block-form kernel (pivoting inside 32 x 32 diagonal
  * blocks, every update on the tensor cores, two 256-thread CTAs per SM; mixed form only); ctas_per_sm: CTAs per
- * SM of the 128-thread kernel (0 = all that fit).  The choices change the speed only: every choice computes the
+ * SM of kernel 2 (0 = all that fit).  The choices change the speed only: every choice computes the
  * same solves (the mixed ones to the refinement tolerance). */
 typedef struct {
   int kernel;
@@ -187,7 +188,7 @@ typedef struct {
 /* Ladder BSE of several requests in ONE persistent launch (the serving path's continuous batch; the upstream
  * runs one create_auxiliary_chi_r_q_sum call per request, dgamore/nonlocal_sde.py:85-156).  Requests may differ
  * in niv, niw, Q, beta, inputs and n_orb (1..4), but every request must take the same default kernel
- * (dga_bse_default_kernel).  The 128-thread kernels (the FP64 form) and the mixed form's block kernel for 1 to 3
+ * (dga_bse_default_kernel).  The FP64 and 128-thread kernels and the mixed form's block kernel for 1 to 3
  * orbitals choose the right-hand-side count per item, so their requests share a launch whatever their orbital
  * counts; the shared-memory-panel kernels and the 4-orbital block kernel take one n_orb per launch.
  * probs_host: the descriptors on the host (launch
