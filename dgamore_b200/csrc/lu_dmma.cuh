@@ -208,14 +208,17 @@ __device__ void lu_block_row(const double2* __restrict__ A, int N, int ld, int j
       const size_t d1 = (size_t)(min(c0 + 8 + g, ncols - 1) - min(c0 + g, ncols - 1)) * ldy;
       int left = k1 - k0 - t;  // rows of Y from this lane's on; past the end they count as zero
       __syncwarp();  // the ring shares its memory with the previous tile's columns
+      // only what a step will wait for: a copy still on its way after the last step would land in the columns below
 #pragma unroll
       for (int u = 0; u < LU_RING - 1; ++u) {
-        const bool in = left > 0;
-        cp_async16_or_zero(&ring[u][0][lane], in ? pb : Y, in);
-        cp_async16_or_zero(&ring[u][1][lane], in ? pb + d1 : Y, in);
+        if (u < steps) {
+          const bool in = left > 0;
+          cp_async16_or_zero(&ring[u][0][lane], in ? pb : Y, in);
+          cp_async16_or_zero(&ring[u][1][lane], in ? pb + d1 : Y, in);
+          pb += 4;
+          left -= 4;
+        }
         cp_async_commit();
-        pb += 4;
-        left -= 4;
       }
       int ra[2 * MT], ca = k0 + t;
 #pragma unroll
