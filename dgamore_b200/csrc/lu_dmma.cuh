@@ -59,6 +59,7 @@ struct LuSmem {
   double2 us[8][NB];               // panel: rows of U of the columns just factored
   double2 cand[2][NT / 32][10];    // panel: each warp's candidate pivot row, conj(pivot), 1 / |pivot|^2
   __align__(16) unsigned long long key[2][(NT / 32 + 1) / 2 * 2];
+  int at[2][NT / 32];              // its position
   int flag;
 };
 
@@ -304,13 +305,12 @@ __device__ __forceinline__ double2 cdot4(int n, FA a, FB b) {
 
 constexpr unsigned long long LU_INF_BITS = 0x7ff0000000000000ull;
 
-// Pivot candidates are compared as one 64-bit integer: the high 48 bits of |re| + |im| (a non-negative double orders as
-// an integer does), then the position, the first one largest, then the warp that offers it. Integers keep the search off
-// the FP64 pipe, where each comparison would wait behind the products of the other warps; entries that agree to 2^-36 are
-// tied and the first of them is taken. 0: no candidate (a NaN is none).
-__device__ __forceinline__ unsigned long long lu_key(double2 a, int pos, int warp) {
+// Pivot candidates are compared as integers: the 64 bits of |re| + |im| (a non-negative double orders as an integer does)
+// plus one, then the position, the first one largest, as LAPACK takes them. Integers keep the search off the FP64 pipe,
+// where each comparison would wait behind the products of the other warps. 0: no candidate (a NaN is none).
+__device__ __forceinline__ unsigned long long lu_key(double2 a) {
   const unsigned long long x = __double_as_longlong(cabs1(a));
-  return x > LU_INF_BITS ? 0 : (x & ~0xffffull) | (unsigned)((2048 - pos) << 4) | (unsigned)warp;
+  return x > LU_INF_BITS ? 0 : x + 1;
 }
 
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long key) {
@@ -426,12 +426,14 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
       if (jj < pw) {
         const int j = jc + jj, buf = jj & 1;
         unsigned long long own = 0;
+        int at = N;
         double2 d = make_double2(0.0, 0.0);
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
-          const unsigned long long x = (pos[i] >= j && pos[i] < N) ? lu_key(a[i][0], pos[i], warp) : 0;
-          if (x > own) {
+          const unsigned long long x = (pos[i] >= j && pos[i] < N) ? lu_key(a[i][0]) : 0;
+          if (x > own || (x == own && pos[i] < at)) {
             own = x;
+            at = pos[i];
             d = a[i][0];
           }
         }
@@ -439,30 +441,38 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
         double rs;
         pivot_recip(d, rc, rs);
         unsigned long long key = warp_max(own);
-        if (own == key && key) {
-          const int p = 2048 - (int)((key >> 4) & 0xfff);
+        bool offer = own == key;
+        if (__popc(__ballot_sync(0xffffffffu, offer)) > 1) {  // a tie: the first row (the whole warp takes the reduction)
+          const unsigned first = __reduce_min_sync(0xffffffffu, offer ? (unsigned)at : 0xffffffffu);
+          offer = (unsigned)at == first;
+        }
+        if (offer && key) {
 #pragma unroll
           for (int i = 0; i < RPT; ++i)
-            if (pos[i] == p) {
+            if (pos[i] == at) {
 #pragma unroll
               for (int c = 0; c < PW; ++c) sm.cand[buf][warp][c] = a[i][c];
             }
           sm.cand[buf][warp][8] = rc;
           sm.cand[buf][warp][9].x = rs;
+          sm.at[buf][warp] = at;
         }
         if (lane == 0) sm.key[buf][warp] = key;
         __syncthreads();
+        int p = sm.at[buf][0], win = 0;
         if constexpr (NW > 1) {
-          const ulonglong2* keys = reinterpret_cast<const ulonglong2*>(sm.key[buf]);
-          key = 0;
+          key = sm.key[buf][0];
 #pragma unroll
-          for (int w = 0; w < NW / 2; ++w) {
-            const ulonglong2 x = keys[w];
-            const unsigned long long m = x.x > x.y ? x.x : x.y;
-            key = m > key ? m : key;
+          for (int w = 1; w < NW; ++w) {
+            const unsigned long long x = sm.key[buf][w];
+            const int q = sm.at[buf][w];
+            if (x > key || (x == key && q < p)) {
+              key = x;
+              p = q;
+              win = w;
+            }
           }
         }
-        int p = 2048 - (int)((key >> 4) & 0xfff), win = (int)(key & 15);
         if (key == 0) {  // no comparable entry (every one is NaN): the diagonal row stays
           p = j;
           win = 0;
