@@ -146,22 +146,23 @@ __global__ void eli_ladder_term_kernel(const double2* __restrict__ uv, const dou
 // Threads of an FP64 CTA: one warp up to N = 64 (29,600 factorisations of N = 40: 1.45 ms, 1.79 with two warps), two up to
 // N = 192 (14,208 of N = 120: 6.8 ms, 7.6 with four), four up to N = 512 (1,184 of N = 480: 18.4 ms, 19.6 with eight), eight
 // above (592 of N = 720: 27.9 ms). Where the items would fill less than half of the SMs' threads that way, each gets more,
-// up to two rows a thread (441 items of N = 200: 1.8 ms with four warps, 2.5 with two).
-static int fp64_threads(int N, int n_items) {
+// up to two rows a thread (441 items of N = 200: 1.8 ms with four warps, 2.5 with two). at_once: the items, or where the
+// launch has room for fewer CTAs (scratch slots, a limit of the caller's), as many as it has room for.
+static int fp64_threads(int N, int at_once) {
   int nt = N <= 64 ? 32 : N <= LU_SMALL_N ? 64 : N <= 512 ? 128 : 256;
-  while (nt < 256 && nt < N && (long)n_items * nt <= (long)device_sm_count() * 256) nt *= 2;
+  while (nt < 256 && nt < N && (long)at_once * nt <= (long)device_sm_count() * 256) nt *= 2;
   return nt;
 }
 }  // namespace dga
 
 using namespace dga;
 
-// Calls f with the FP64 kernels' thread count for n_items items of sizes up to N as a compile-time constant, and their
+// Calls f with the FP64 kernels' thread count for sizes up to N (fp64_threads) as a compile-time constant, and their
 // dynamic shared memory.
 template <typename F>
-static auto with_fp64_threads(int N, int n_items, F f) {
+static auto with_fp64_threads(int N, int at_once, F f) {
   const size_t piv = sizeof(int) * (size_t)N;
-  switch (fp64_threads(N, n_items)) {
+  switch (fp64_threads(N, at_once)) {
     case 32: return f(std::integral_constant<int, 32>{}, sizeof(Fp64Smem<32>) + piv);
     case 64: return f(std::integral_constant<int, 64>{}, sizeof(Fp64Smem<64>) + piv);
     case 128: return f(std::integral_constant<int, 128>{}, sizeof(Fp64Smem<128>) + piv);
@@ -189,23 +190,30 @@ static int grid_for(K kernel, int n_items, size_t smem, int threads = BSE_THREAD
   return n_items < g ? n_items : g;
 }
 
-static int bse_grid(int N, int n_items) {
-  return with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
-    return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, nt.value>, n_items, smem, nt.value);
-  });
+// An FP64 launch over n_items items by at most `limit` CTAs.
+struct Fp64Run {
+  int at_once, grid;
+};
+
+static Fp64Run bse_run(int N, int n_items, size_t limit = (size_t)-1) {
+  const int at_once = (size_t)n_items < limit ? n_items : (int)limit;
+  return {at_once, with_fp64_threads(N, at_once, [&](auto nt, size_t smem) {
+            return grid_for(bse_solve_sum_fp64_kernel<StructuredSource, nt.value>, at_once, smem, nt.value);
+          })};
 }
 
 static bool supported_rhs(int n2) { return n2 == 1 || n2 == 4 || n2 == 9 || n2 == 16; }
 
 template <typename Source>
-static void launch_fp64(int n2, int grid, cudaStream_t stream, const Source& src, const WorkItem* work, int n_items,
+static void launch_fp64(int n2, Fp64Run run, cudaStream_t stream, const Source& src, const WorkItem* work, int n_items,
                         int N, int nv, int W, int Q, double beta, double2* out, int* status, double2* scratch,
                         size_t slot, int redo) {
-  with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
+  with_fp64_threads(N, run.at_once, [&](auto nt, size_t smem) {
     auto kernel = bse_solve_sum_fp64_kernel<Source, nt.value>;
-    prepare_kernel(kernel, smem, nt.value);
-    kernel<<<grid, nt.value, smem, stream>>>(src, work, n_items, N, n2, nv, W, Q, beta, out, status, scratch, slot,
-                                             redo);
+    // bse_run has set the structured kernel's limits
+    if constexpr (!std::is_same_v<Source, StructuredSource>) prepare_kernel(kernel, smem, nt.value);
+    kernel<<<run.grid, nt.value, smem, stream>>>(src, work, n_items, N, n2, nv, W, Q, beta, out, status, scratch, slot,
+                                                 redo);
   });
 }
 
@@ -215,8 +223,7 @@ extern "C" {
 // n2 right-hand sides: one N x N matrix plus N x n2 solution per resident CTA.
 size_t dga_bse_scratch_bytes(int N, int n2, int n_items) {
   if (N <= 0 || n2 <= 0 || n_items <= 0) return 0;
-  const int grid = bse_grid(N, n_items);
-  return (size_t)grid * ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
+  return (size_t)bse_run(N, n_items).grid * ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
 }
 
 int dga_bse_solve_sum_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, double beta, double inv_beta2,
@@ -233,11 +240,11 @@ int dga_bse_solve_sum_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, 
     dga_set_error("dga_bse_solve_sum_c128: null pointer argument");
     return DGA_ERR_ARG;
   }
-  const int grid = bse_grid(N, n_items);
+  const Fp64Run run = bse_run(N, n_items);
   const size_t slot = (size_t)N * N + (size_t)N * n2;
-  if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
+  if (scratch_bytes < (size_t)run.grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_solve_sum_c128: scratch too small (%zu < %zu)", scratch_bytes,
-                  (size_t)grid * slot * sizeof(double2));
+                  (size_t)run.grid * slot * sizeof(double2));
     return DGA_ERR_SCRATCH;
   }
   StructuredSource src;
@@ -249,7 +256,7 @@ int dga_bse_solve_sum_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, 
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, run, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -272,10 +279,9 @@ int dga_bse_resolve_fp64_c128(int n_orb, int niv, int niw_half, int n_q, int n_c
     dga_set_error("dga_bse_resolve_fp64_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  int grid = bse_grid(N, n_items);
-  if (grid > grid_limit) grid = grid_limit;
+  const Fp64Run run = bse_run(N, n_items, (size_t)grid_limit);
   const size_t slot = (size_t)N * N + (size_t)N * n2;
-  if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
+  if (scratch_bytes < (size_t)run.grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_resolve_fp64_c128: scratch too small");
     return DGA_ERR_SCRATCH;
   }
@@ -288,7 +294,7 @@ int dga_bse_resolve_fp64_c128(int n_orb, int niv, int niw_half, int n_q, int n_c
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, run, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 1);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -309,9 +315,9 @@ int dga_invert_sum_dense_c128(int n_orb, int niv, int niw_half, int n_q, double 
     dga_set_error("dga_invert_sum_dense_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const int grid = bse_grid(N, n_items);
+  const Fp64Run run = bse_run(N, n_items);
   const size_t slot = (size_t)N * N + (size_t)N * n2;
-  if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
+  if (scratch_bytes < (size_t)run.grid * slot * sizeof(double2)) {
     dga_set_error("dga_invert_sum_dense_c128: scratch too small");
     return DGA_ERR_SCRATCH;
   }
@@ -321,7 +327,7 @@ int dga_invert_sum_dense_c128(int n_orb, int niv, int niw_half, int n_q, double 
   src.nv = nv;
   src.W = niw_half;
   src.Q = n_q;
-  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, run, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
@@ -575,18 +581,19 @@ static size_t batch_smem(int n_max, int n2, int mixed) {
   return mixed ? mixed_smem_bytes(n_max, n2) : 0;  // the FP64 kernels' own: with_fp64_threads
 }
 
-// The batch kernels' grids for requests of sizes up to n_max (n2 = 0: of several orbital counts).
-static int batch_grid(int mixed, int n2, int n_max, int n_items, size_t smem) {
+// The batch kernels' grids for requests of sizes up to n_max (n2 = 0: of several orbital counts); at_once: the items or the
+// scratch slots, whichever are fewer.
+static int batch_grid(int mixed, int n2, int n_max, int at_once, size_t smem) {
   if (!mixed)
-    return with_fp64_threads(n_max, n_items, [&](auto nt, size_t smem64) {
-      return grid_for(bse_multi_fp64_kernel<nt.value>, n_items, smem64, nt.value);
+    return with_fp64_threads(n_max, at_once, [&](auto nt, size_t smem64) {
+      return grid_for(bse_multi_fp64_kernel<nt.value>, at_once, smem64, nt.value);
     });
   switch (n2) {
-    case 0: return grid_for(bse_multi_mixed_kernel<0>, n_items, smem);
-    case 1: return grid_for(bse_multi_mixed_kernel<1>, n_items, smem);
-    case 4: return grid_for(bse_multi_mixed_kernel<4>, n_items, smem);
-    case 9: return grid_for(bse_multi_mixed_kernel<9>, n_items, smem);
-    case 16: return grid_for(bse_multi_mixed_kernel<16>, n_items, smem);
+    case 0: return grid_for(bse_multi_mixed_kernel<0>, at_once, smem);
+    case 1: return grid_for(bse_multi_mixed_kernel<1>, at_once, smem);
+    case 4: return grid_for(bse_multi_mixed_kernel<4>, at_once, smem);
+    case 9: return grid_for(bse_multi_mixed_kernel<9>, at_once, smem);
+    case 16: return grid_for(bse_multi_mixed_kernel<16>, at_once, smem);
     default: return 0;
   }
 }
@@ -643,14 +650,15 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
   const int n2 = probs_host[0].n_orb * probs_host[0].n_orb;
   const size_t smem = batch_smem(n_max, hetero ? n2_max : n2, mixed);
   const bool panel = kernel != 2;
-  int grid = panel    ? (kernel == 4 ? dga_block_grid(hetero ? 0 : n2, n_items)
-                                     : dga_panel_batch_grid(n2, n_max, n_items, kernel == 3))
-                      : batch_grid(mixed, hetero ? 0 : n2, n_max, n_items, smem);
   if (scratch_bytes < slot) {
     dga_set_error("dga_bse_solve_sum_batch_c128: scratch too small (%zu < one slot of %zu)", scratch_bytes, slot);
     return DGA_ERR_SCRATCH;
   }
-  if ((size_t)grid > scratch_bytes / slot) grid = (int)(scratch_bytes / slot);
+  const int at_once = (size_t)n_items < scratch_bytes / slot ? n_items : (int)(scratch_bytes / slot);
+  int grid = panel    ? (kernel == 4 ? dga_block_grid(hetero ? 0 : n2, n_items)
+                                     : dga_panel_batch_grid(n2, n_max, n_items, kernel == 3))
+                      : batch_grid(mixed, hetero ? 0 : n2, n_max, at_once, smem);
+  if (grid > at_once) grid = at_once;
   const int redo = mode == 2;
   const dga_bse_problem* pd = (const dga_bse_problem*)probs_dev;
   const MultiItem* wk = (const MultiItem*)work;
@@ -679,7 +687,7 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
       case 16: go(bse_multi_mixed_kernel<16>); break;
     }
   } else {
-    with_fp64_threads(n_max, n_items, [&](auto nt, size_t smem64) {
+    with_fp64_threads(n_max, at_once, [&](auto nt, size_t smem64) {
       bse_multi_fp64_kernel<nt.value><<<grid, nt.value, smem64, stream>>>(pd, wk, n_items, n_max, status, iters, sc, slot,
                                                                         redo);
     });
@@ -727,8 +735,9 @@ static int tuned_kernel(int mixed, int N, int n2, const dga_bse_tuning* t) {
   return k;
 }
 
+// run: the FP64 form's threads and grid (the returned grid again)
 static int tuned_grid(int kernel, int mixed, int N, int n2, int n_items, const dga_bse_tuning* t, size_t* slot,
-                      size_t* smem) {
+                      size_t* smem, Fp64Run* run) {
   if (kernel == 1 || kernel == 3) {
     *slot = dga_panel_slot_bytes(N, n2);
     *smem = 0;
@@ -739,22 +748,18 @@ static int tuned_grid(int kernel, int mixed, int N, int n2, int n_items, const d
     *smem = 0;
     return dga_block_grid(n2, n_items);
   }
-  int grid;
-  if (mixed) {
-    *smem = mixed_smem_bytes(N, n2);
-    *slot = mixed_slot_bytes(N, n2);
-    grid = mixed_grid(n_items, *smem);
-  } else {
+  const int cps = t ? t->ctas_per_sm : 0;
+  const size_t cap = cps > 0 ? (size_t)sm_count() * cps : (size_t)-1;
+  if (!mixed) {
     *smem = 0;  // with_fp64_threads
     *slot = ((size_t)N * N + (size_t)N * n2) * sizeof(double2);
-    grid = bse_grid(N, n_items);
+    *run = bse_run(N, n_items, cap);
+    return run->grid;
   }
-  const int cps = t ? t->ctas_per_sm : 0;
-  if (cps > 0) {
-    const int cap = sm_count() * cps;
-    if (grid > cap) grid = cap;
-  }
-  return grid;
+  *smem = mixed_smem_bytes(N, n2);
+  *slot = mixed_slot_bytes(N, n2);
+  const int grid = mixed_grid(n_items, *smem);
+  return (size_t)grid > cap ? (int)cap : grid;
 }
 
 extern "C" {
@@ -764,7 +769,9 @@ size_t dga_bse_tuned_scratch_bytes(int N, int n2, int n_items, int mixed, const 
   const int kernel = tuned_kernel(mixed, N, n2, t);
   if (kernel < 0) return 0;
   size_t slot = 0, smem = 0;
-  return (size_t)tuned_grid(kernel, mixed, N, n2, n_items, t, &slot, &smem) * slot;
+  Fp64Run run{};
+  const int grid = tuned_grid(kernel, mixed, N, n2, n_items, t, &slot, &smem, &run);
+  return (size_t)grid * slot;
 }
 
 int dga_bse_solve_sum_tuned_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, double beta, double inv_beta2,
@@ -788,7 +795,8 @@ int dga_bse_solve_sum_tuned_c128(int n_orb, int niv, int niw_half, int n_q, int 
     return DGA_ERR_ARG;
   }
   size_t slot = 0, smem = 0;
-  const int grid = tuned_grid(kernel, mixed, N, n2, n_items, t, &slot, &smem);
+  Fp64Run run{};
+  const int grid = tuned_grid(kernel, mixed, N, n2, n_items, t, &slot, &smem, &run);
   if (scratch_bytes < (size_t)grid * slot) {
     dga_set_error("dga_bse_solve_sum_tuned_c128: scratch too small (%zu < %zu)", scratch_bytes, (size_t)grid * slot);
     return DGA_ERR_SCRATCH;
@@ -827,7 +835,7 @@ int dga_bse_solve_sum_tuned_c128(int n_orb, int niv, int niw_half, int n_q, int 
 #undef DGA_TUNED_MIXED_CASE
     err = cudaGetLastError();
   } else {
-    launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+    launch_fp64(n2, run, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
                 (double2*)out, status, (double2*)scratch, slot / sizeof(double2), 0);
     err = cudaGetLastError();
   }
@@ -916,8 +924,7 @@ int dga_bse_solve_sum_noalloc_c128(int n_orb, int niv, int niw_half, int n_q, in
   void* scratch = nullptr;
   int rc = noalloc_scratch_ptr(&scratch);
   if (rc != DGA_OK) return rc;
-  int grid = bse_grid(N, n_items);
-  if ((size_t)grid > capacity_slots) grid = (int)capacity_slots;
+  const Fp64Run run = bse_run(N, n_items, capacity_slots);
   StructuredSource src;
   src.gamma_cm = (const double2*)gamma_cm;
   src.chi0_inv = (const double2*)chi0_inv;
@@ -927,7 +934,7 @@ int dga_bse_solve_sum_noalloc_c128(int n_orb, int niv, int niw_half, int n_q, in
   src.W = niw_half;
   src.Q = n_q;
   src.inv_beta2 = inv_beta2;
-  launch_fp64(n2, grid, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
+  launch_fp64(n2, run, stream, src, (const WorkItem*)work, n_items, N, nv, niw_half, n_q, beta,
               (double2*)out, status, (double2*)scratch, slot, 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
