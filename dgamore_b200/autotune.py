@@ -103,7 +103,8 @@ def tune_bse(lp, precision: str | None = None, sample_items: int | None = None, 
     sms = torch.cuda.get_device_properties(lp.dev).multi_processor_count
     n = lp.n_items if sample_items is None else min(lp.n_items, sample_items)
     if sample_items is None:
-        n = min(lp.n_items, 6 * sms)
+        # more than eight per SM: a shorter list would get more threads an FP64 CTA than the whole one
+        n = min(lp.n_items, 9 * sms)
     work = lp.work[:n].contiguous()
     status = torch.zeros(n, dtype=torch.int32, device=lp.dev)
     iters = torch.zeros(n, dtype=torch.int32, device=lp.dev)
