@@ -160,6 +160,19 @@ inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 // SMs of the current device (cached per device; 148 on B200).
 int device_sm_count();
+// Shared memory a CTA may ask for on the current device (cached per device; 227 KB on B200).
+int device_max_shared_memory();
+
+// Lets a kernel take all the dynamic shared memory that a CTA can have. The limit is the kernel's, not the launch's, and
+// so always the same value: with each launch's own size, a thread could lower it between another's call and its launch.
+// Occupancy and the L1 split follow what a launch asks for.
+template <typename K>
+inline void allow_shared_memory(K* kernel) {
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess)
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         device_max_shared_memory() - (int)a.sharedSizeBytes);
+}
 
 }  // namespace dga
 

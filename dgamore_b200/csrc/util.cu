@@ -32,6 +32,18 @@ int device_sm_count() {
   return sms;
 }
 
+int device_max_shared_memory() {
+  static int cache[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 227 * 1024;
+  if (dev < 64 && cache[dev] > 0) return cache[dev];
+  int bytes = 0;
+  if (cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || bytes <= 0)
+    bytes = 227 * 1024;
+  if (dev < 64) cache[dev] = bytes;
+  return bytes;
+}
+
 }  // namespace dga
 
 extern "C" int dga_device_sm_count(void) { return dga::device_sm_count(); }

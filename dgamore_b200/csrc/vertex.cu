@@ -606,7 +606,7 @@ int dga_chi0_prep_c128(const void* chi0, int n_orb, int niv_core, int niv_shell,
   const long long n_mats = (long long)n_q * niw_half * nv;
   const int th = small_threads(n2);
   const size_t smem = (size_t)th * n2 * n2 * sizeof(double2);
-  cudaFuncSetAttribute(chi0_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared_memory(chi0_inverse_kernel);
   chi0_inverse_kernel<<<(int)((n_mats + th - 1) / th), th, smem, stream>>>(
       (const double2*)chi0, n2, nvf, nv, niv_shell, n_mats, (double2*)chi0_inv, status);
   if (vstatus("dga_chi0_prep_c128")) return DGA_ERR_LAUNCH;
@@ -647,7 +647,7 @@ int dga_lambda_c128(const void* chi, int n_q, int niw_half, int n_ch, const long
   }
   const long long per = ((long long)n_q * niw_half + LAMBDA_CTAS - 1) / LAMBDA_CTAS;
   const size_t smem = (size_t)(per < LAMBDA_CACHED ? per : LAMBDA_CACHED) * sizeof(double2);
-  cudaFuncSetAttribute(lambda_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared_memory(lambda_kernel);
   lambda_kernel<<<n_ch * LAMBDA_CTAS, LAMBDA_THREADS, smem, stream>>>((const double2*)chi, n_q, niw_half, weights,
                                                                       (const double2*)target, beta, nk_tot, delta, eps,
                                                                       maxiter, lambda_out, iters_out, status,
@@ -669,7 +669,7 @@ int dga_kernel_assembly_c128(const void* chi0_inv, const void* X, const void* uv
   const int blocks = (int)((total + per_block - 1) / per_block);
 #define DGA_KA_CASE(NN)                                                                                        \
   case NN:                                                                                                     \
-    cudaFuncSetAttribute(kernel_assembly_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+    allow_shared_memory(kernel_assembly_kernel<NN>);                                                           \
     kernel_assembly_kernel<NN><<<blocks, 32 * KA_WARPS, smem, stream>>>(                                       \
         (const double2*)chi0_inv, (const double2*)X, (const double2*)uv, (const double2*)chi_phys,             \
         (const double2*)k_dc, 2 * niv_core, niw_half, n_q, beta, (double2*)K, (double2*)gamma_out);            \
@@ -712,7 +712,7 @@ int dga_dc_kernel_c128(const void* chi0, const void* u_perm, const void* fdc, in
     return DGA_ERR_ARG;
   }
   const size_t left_smem = (size_t)nus * ((n2 * n2) | 1) * sizeof(double2);
-  cudaFuncSetAttribute(dc_left_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)left_smem);
+  allow_shared_memory(dc_left_kernel);
   dc_left_kernel<<<(int)left_blocks, 256, left_smem, stream>>>(
       (const double2*)chi0, (const double2*)u_perm, n2, n_q, niw_half, nvf, nus, (double2*)scratch);
   if (vstatus("dga_dc_kernel_c128")) return DGA_ERR_LAUNCH;
