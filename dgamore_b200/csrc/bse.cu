@@ -702,9 +702,16 @@ int dga_bse_solve_sum_batch_c128(const dga_bse_problem* probs_host, const void* 
 
 }  // extern "C"
 
-// Loads the code of the block-form BSE kernels ahead of their first launch (see include/dga_b200.h).
+// Loads the code of a batch's kernels ahead of their first launch (see include/dga_b200.h): the block form's and the FP64
+// kernels of every thread count, since which of them a batch takes changes with its sizes (2.4 to 10 ms at a first use).
 extern "C" int dga_bse_preload(void) {
-  if (dga_block_preload()) {
+  cudaFuncAttributes a;
+  int bad = dga_block_preload();
+  bad |= cudaFuncGetAttributes(&a, bse_multi_fp64_kernel<32>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, bse_multi_fp64_kernel<64>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, bse_multi_fp64_kernel<128>) != cudaSuccess;
+  bad |= cudaFuncGetAttributes(&a, bse_multi_fp64_kernel<256>) != cudaSuccess;
+  if (bad) {
     dga_set_error("dga_bse_preload: a kernel could not be loaded: %s", cudaGetErrorString(cudaGetLastError()));
     return DGA_ERR_LAUNCH;
   }
