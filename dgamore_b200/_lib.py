@@ -62,6 +62,7 @@ SIGNATURES = {
     "dga_sigma_kmean_c128": (I, [VP, I, I, I, I, I, VP, VP]),
     "dga_bse_solve_sum_tuned_c128": (I, [I, I, I, I, I, D, D, VP, VP, VP, PI, I, I, I, D, VP, PI, PI, VP, VP, SZ, VP]),
     "dga_bse_eli_scratch_bytes": (SZ, [I, I, I]),
+    "dga_bse_eli_box_scratch_bytes": (SZ, [I, I, I, I]),
     "dga_bse_solve_sum_eli_c128": (I, [I, I, I, I, I, D, D, VP, VP, VP, PI, I, I, I, VP, VP, PI, VP, SZ, VP]),
     "dga_eli_ladder_term_c128": (I, [VP, VP, VP, I, I, I, I, I, I, VP, VP]),
     "dga_sigma_wedge_scratch_bytes": (SZ, [I, I, I, I, I, I]),

@@ -1009,8 +1009,8 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
 
 }  // extern "C"
 
-// Scratch of one CTA of the fused form: the matrix, the selectors and the box columns, at most N of them (niv_pp <= niv).
-static size_t eli_fused_slot(int N, int n2) { return (size_t)N * N + (size_t)N * n2 + (size_t)N * N; }
+// Scratch of one CTA of the fused form: the matrix, the selectors and the box columns.
+static size_t eli_fused_slot(int N, int n2, int niv_pp) { return (size_t)N * (N + n2 + (size_t)n2 * 2 * niv_pp); }
 
 static int eli_grid(int N, int n_items) {
   return with_fp64_threads(N, n_items, [&](auto nt, size_t smem) {
@@ -1020,11 +1020,16 @@ static int eli_grid(int N, int n_items) {
 
 extern "C" {
 
-// Scratch bytes of dga_bse_solve_sum_eli_c128 for n_items items of size N.
+// Scratch bytes of dga_bse_solve_sum_eli_c128 for n_items items of size N with a box of niv_pp frequencies.
+size_t dga_bse_eli_box_scratch_bytes(int N, int n2, int niv_pp, int n_items) {
+  if (N <= 0 || !supported_rhs(n2) || niv_pp <= 0 || n_items <= 0) return 0;
+  return (size_t)eli_grid(N, n_items) * eli_fused_slot(N, n2, niv_pp) * sizeof(double2);
+}
+
+// The same for the largest box (niv_pp = niv, N columns).
 size_t dga_bse_eli_scratch_bytes(int N, int n2, int n_items) {
   if (N <= 0 || !supported_rhs(n2) || n_items <= 0) return 0;
-  const int grid = eli_grid(N, n_items);
-  return (size_t)grid * eli_fused_slot(N, n2) * sizeof(double2);
+  return dga_bse_eli_box_scratch_bytes(N, n2, (N + 2 * n2 - 1) / (2 * n2), n_items);
 }
 
 // dga_bse_solve_sum_c128 whose items with w < w_pp also write the chi* part of the Eliashberg full vertex in the pp
@@ -1041,7 +1046,7 @@ int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_
     dga_set_error("dga_bse_solve_sum_eli_c128: invalid arguments");
     return DGA_ERR_ARG;
   }
-  const size_t slot = eli_fused_slot(N, n2);
+  const size_t slot = eli_fused_slot(N, n2, niv_pp);
   const int grid = eli_grid(N, n_items);
   if (scratch_bytes < (size_t)grid * slot * sizeof(double2)) {
     dga_set_error("dga_bse_solve_sum_eli_c128: scratch too small");

@@ -320,7 +320,8 @@ class LadderPass:
             # the BSE runs in a batch launch (serving.solve_bse_batch) that brings its own scratch
             self.bse_scratch = self.mixed_scratch = None
         elif precision == "fp64" and eliashberg_pp:
-            self.bse_scratch_bytes = int(lib().dga_bse_eli_scratch_bytes(N, n2, self.n_items))
+            box = min(int(eliashberg_pp), sh.niv)
+            self.bse_scratch_bytes = int(lib().dga_bse_eli_box_scratch_bytes(N, n2, box, self.n_items))
         elif precision == "fp64":
             self.bse_scratch_bytes = int(lib().dga_bse_scratch_bytes(N, n2, self.n_items))
         else:

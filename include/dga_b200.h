@@ -318,8 +318,10 @@ int dga_eli_full_vertex_c128(int n_orb, int niv, int niw_half, int n_q, int niv_
  * out_pp [2][Q][w_pp][Mb][Mb] = beta^2 (delta c0 - c0 chi* c0), the chi* part of the vertex of
  * create_full_vertex_q_r(_v2) (dgamore/eliashberg_solver.py:78-298), without a second factorisation.
  * dga_eli_ladder_term_c128 adds the ladder term (U_r - U_r chi_r U_r) gamma_r gamma_r once the pass has the
- * lambda-corrected chi_r and the three-leg vertex, giving the out of dga_eli_full_vertex_c128. */
-size_t dga_bse_eli_scratch_bytes(int N, int n2, int n_items);
+ * lambda-corrected chi_r and the three-leg vertex, giving the out of dga_eli_full_vertex_c128.  Scratch: one N x
+ * (N + n2 + 2 niv_pp n2) matrix of complex128 per resident CTA. */
+size_t dga_bse_eli_box_scratch_bytes(int N, int n2, int niv_pp, int n_items);
+size_t dga_bse_eli_scratch_bytes(int N, int n2, int n_items); /* for a box of any size */
 int dga_bse_solve_sum_eli_c128(int n_orb, int niv, int niw_half, int n_q, int n_ch, double beta, double inv_beta2,
                                const void* gamma_cm, const void* chi0_inv, const void* uv, const int* work,
                                int n_items, int niv_pp, int w_pp, void* out, void* out_pp, int* status, void* scratch,
