@@ -174,7 +174,7 @@ static auto with_fp64_threads(int N, int at_once, F f) {
 // carve-out the driver may size shared memory for fewer CTAs than fit (six of eight for the two-warp FP64 kernel).
 template <typename K>
 static int prepare_kernel(K kernel, size_t smem, int threads) {
-  allow_shared_memory(kernel);
+  allow_shared_memory(kernel, smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (per_sm < 1) per_sm = 1;
@@ -437,7 +437,7 @@ int dga_bse_solve_sum_mixed_c128(int n_orb, int niv, int niw_half, int n_q, int 
   }
 #define DGA_MIXED_CASE(NRV)                                                                                       \
   case NRV:                                                                                                       \
-    allow_shared_memory(bse_solve_sum_mixed_kernel<NRV>);                                                          \
+    allow_shared_memory(bse_solve_sum_mixed_kernel<NRV>, smem);                                                    \
     bse_solve_sum_mixed_kernel<NRV><<<grid, BSE_THREADS, smem, stream>>>(                                          \
         src, (const WorkItem*)work, n_items, N, NRV, nv, niw_half, n_q, beta, max_iter, tol, (double2*)out, status, \
         iters, (unsigned char*)scratch, slot);                                                                    \
@@ -828,7 +828,7 @@ int dga_bse_solve_sum_tuned_c128(int n_orb, int niv, int niw_half, int n_q, int 
   } else if (mixed) {
 #define DGA_TUNED_MIXED_CASE(NRV)                                                                                    \
   case NRV:                                                                                                          \
-    allow_shared_memory(bse_solve_sum_mixed_kernel<NRV>);                                                            \
+    allow_shared_memory(bse_solve_sum_mixed_kernel<NRV>, smem);                                                      \
     bse_solve_sum_mixed_kernel<NRV><<<grid, BSE_THREADS, smem, stream>>>(                                            \
         src, (const WorkItem*)work, n_items, N, NRV, nv, niw_half, n_q, beta, max_iter, tol, (double2*)out, status,  \
         iters, (unsigned char*)scratch, slot);                                                                       \
@@ -1086,7 +1086,7 @@ int dga_eli_ladder_term_c128(const void* uv, const void* g3, const void* chi_phy
     return DGA_ERR_ARG;
   }
   const size_t smem = ((size_t)n2 * n2 + (size_t)2 * niv_pp * n2 * n2) * sizeof(double2);
-  allow_shared_memory(eli_ladder_term_kernel);
+  allow_shared_memory(eli_ladder_term_kernel, smem);
   eli_ladder_term_kernel<<<2 * n_q * w_pp, 256, smem, stream>>>((const double2*)uv, (const double2*)g3,
                                                               (const double2*)chi_phys, n2, nv, niw_half, n_q,
                                                               niv_pp, w_pp, (double2*)f);

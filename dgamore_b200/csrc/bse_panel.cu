@@ -987,7 +987,7 @@ static int panel_grid_for(K kernel, int n_items, size_t smem) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  allow_shared_memory(kernel);
+  allow_shared_memory(kernel, smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, PT, smem);
   if (per_sm < 1) per_sm = 1;

@@ -688,7 +688,7 @@ int dga_dft_planes_c128(const void* in, long long in_s_hi, long long in_s_lo, lo
   const Grid3 g = make_grid(nx, ny, nz);
   PlaneAddr ia{in_s_hi, in_s_lo, in_s_r, n_lo}, oa{out_s_hi, out_s_lo, out_s_r, n_lo};
   const size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
-  allow_shared_memory(dft_planes_kernel);
+  allow_shared_memory(dft_planes_kernel, smem);
   dft_planes_kernel<<<grid_cap(n_planes), plane_threads(g.nk), smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
                                                                       n_planes, g, (const double2*)tw, scale, nullptr);
   return launch_status("dga_dft_planes_c128");
@@ -708,7 +708,7 @@ int dga_dft_planes_gather_c128(const void* in, long long in_s_hi, long long in_s
   const Grid3 g = make_grid(nx, ny, nz);
   PlaneAddr ia{in_s_hi, in_s_lo, in_s_r, n_lo}, oa{out_s_hi, out_s_lo, out_s_r, n_lo};
   const size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
-  allow_shared_memory(dft_planes_kernel);
+  allow_shared_memory(dft_planes_kernel, smem);
   dft_planes_kernel<<<grid_cap(n_planes), plane_threads(g.nk), smem, stream>>>((const double2*)in, ia, (double2*)out, oa,
                                                                       n_planes, g, (const double2*)tw, scale, gather);
   return launch_status("dga_dft_planes_gather_c128");
@@ -734,7 +734,7 @@ int dga_bubble_c128(const void* g_r, int n_orb, int niv, int niw, int nx, int ny
   }
   const size_t smem = (2 * (size_t)g.nk + (size_t)ny * nz + nx + ny + nz) * sizeof(double2) +
                       (6 * (size_t)n_qirr + 1) * sizeof(int);
-  allow_shared_memory(bubble_kernel);
+  allow_shared_memory(bubble_kernel, smem);
   const long long work = (long long)(niw + 1) * 2 * niv * n_orb * n_orb;
   // Four CTAs per resident one: each numbers the (qy, qz) pairs of the q list once, a serial pass that takes longer than a
   // plane at the larger grids (2.95 ms for 561 q of 64 x 64 when every plane's CTA repeated it, 1.44 ms now), and the last
@@ -789,7 +789,7 @@ int dga_sigma_wedge_c128(const void* kern, const void* g_r, int n_orb, int niv, 
   const size_t smem = sizeof(int) * (size_t)g.nk;
   const long long work = (long long)niv * n2 * n_chunks;
   auto partial = [&](auto kernel) {
-    allow_shared_memory(kernel);
+    allow_shared_memory(kernel, smem);
     kernel<<<grid_cap(work), BZ_THREADS, smem, stream>>>(kw, (const double2*)g_r, n_orb, niv, niw, n_q, g.nk,
                                                          irrk_inv, n_chunks, part);
   };
@@ -802,7 +802,7 @@ int dga_sigma_wedge_c128(const void* kern, const void* g_r, int n_orb, int niv, 
                                                                          -0.5 / beta / (double)g.nk, sig);
   if (launch_status("dga_sigma_wedge_c128")) return DGA_ERR_LAUNCH;
   const size_t dsmem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
-  allow_shared_memory(dft_planes_kernel);
+  allow_shared_memory(dft_planes_kernel, dsmem);
   PlaneAddr pa{(long long)g.nk, 0, 1, 1};
   dft_planes_kernel<<<grid_cap(niv * n2), plane_threads(g.nk), dsmem, stream>>>(sig, pa, part, pa, niv * n2, g,
                                                                        (const double2*)tw_inv, 1.0 / (double)g.nk,
@@ -841,7 +841,7 @@ int dga_fbz_rotate_c128(const void* src, const int* irrk_inv, int nk, const void
     return DGA_ERR_ARG;
   }
   const size_t smem = (size_t)fc * n4 * 2 * sizeof(double2);
-  allow_shared_memory(fbz_rotate_kernel);
+  allow_shared_memory(fbz_rotate_kernel, smem);
   fbz_rotate_kernel<<<dim3((unsigned)chunks, nk), BZ_THREADS, smem, stream>>>(
       (const double2*)src, irrk_inv, (const double2*)us, sigmas, conjs, n_orb, L, fc, (double2*)dst);
   return launch_status("dga_fbz_rotate_c128");
@@ -863,7 +863,7 @@ static int sigma_contract(const void* kern, const void* g_r, int n_orb, int niv,
   const size_t smem = (2 * (size_t)g.nk + g.nx + g.ny + g.nz) * sizeof(double2) + sizeof(int) * (size_t)g.nk;
   const long long work = (long long)niv * n2 * n_chunks;
   auto partial = [&](auto kernel) {
-    allow_shared_memory(kernel);
+    allow_shared_memory(kernel, smem);
     kernel<<<grid_cap(work), BZ_THREADS, smem, stream>>>((const double2*)kern, (const double2*)g_r, n_orb, niv, niw,
                                                          n_q, g, irrk_inv, (const double2*)tw_inv, n_chunks, part);
   };
@@ -932,7 +932,7 @@ int dga_sigma_c128(const void* kern, const void* g_r, int n_orb, int niv, int ni
   const long long n_out = (long long)niv * n2 * g.nk;
   // inverse transform over R (normalised 1/Nk), planes contiguous; result back into `part`
   size_t smem = (2 * (size_t)g.nk + nx + ny + nz) * sizeof(double2);
-  allow_shared_memory(dft_planes_kernel);
+  allow_shared_memory(dft_planes_kernel, smem);
   PlaneAddr pa{(long long)g.nk, 0, 1, 1};
   dft_planes_kernel<<<grid_cap(niv * n2), plane_threads(g.nk), smem, stream>>>(sig, pa, part, pa, niv * n2, g,
                                                                       (const double2*)tw_inv, 1.0 / (double)g.nk,

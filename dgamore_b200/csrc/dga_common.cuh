@@ -163,13 +163,14 @@ int device_sm_count();
 // Shared memory a CTA may ask for on the current device (cached per device; 227 KB on B200).
 int device_max_shared_memory();
 
-// Lets a kernel take all the dynamic shared memory that a CTA can have. The limit is the kernel's, not the launch's, and
-// so always the same value: with each launch's own size, a thread could lower it between another's call and its launch.
-// Occupancy and the L1 split follow what a launch asks for.
+// Lets a kernel take the dynamic shared memory of a launch. The limit is the kernel's, not the launch's, and so always
+// raised to the same value, all that a CTA can have: with each launch's own size, a thread could lower it between another's
+// call and its launch. Occupancy and the L1 split follow what a launch asks for. Up to 32 KB (of the 48 KB that need no
+// raising; the rest is left for static arrays) the limit is not looked at, which would be 0.4 us of each short launch.
 template <typename K>
-inline void allow_shared_memory(K* kernel) {
+inline void allow_shared_memory(K* kernel, size_t smem) {
   cudaFuncAttributes a;
-  if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess)
+  if (smem > 32 * 1024 && cudaFuncGetAttributes(&a, kernel) == cudaSuccess)
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          device_max_shared_memory() - (int)a.sharedSizeBytes);
 }

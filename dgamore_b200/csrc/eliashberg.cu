@@ -294,7 +294,7 @@ static int eli_matvec(const char* who, const void* mat, const void* chi0pp, cons
   int rc = dga_dft_planes_c128(s0, 1, 0, M, s1, 1, 0, M, 1, M, nx, ny, nz, tw_fwd, 1.0, stream);
   if (rc) return rc;
   const size_t smem = 2 * (size_t)M * sizeof(double2);
-  allow_shared_memory(eli_vertex_apply_kernel<MT, U, RW>);
+  allow_shared_memory(eli_vertex_apply_kernel<MT, U, RW>, smem);
   const int apply_cap = 8 * device_sm_count();
   eli_vertex_apply_kernel<MT, U, RW><<<nk < apply_cap ? nk : apply_cap, ELI_APPLY_THREADS, smem, stream>>>(
       (const MT*)mat, s1, n_orb, nvp, nk, s2, s3);

@@ -367,7 +367,8 @@ kernel_assembly_kernel(const double2* __restrict__ chi0_inv, const double2* __re
   double2* t1 = g3 + nn;
   double2* t2 = t1 + nn;
   const long long total = (long long)Q * W * nv, mine = blockIdx.x * (long long)(32 * KA_WARPS / GL) + slot;
-  const bool valid = mine < total;  // the others of the warp's matrices go on: its barriers are the warp's
+  if (mine - slot % (32 / GL) >= total) return;  // a warp without a matrix (the block has no block-wide barrier)
+  const bool valid = mine < total;               // the others of a warp's matrices go on: its barriers are the warp's
   const long long t = valid ? mine : total - 1;
   const int v = (int)(t % nv);
   const long long qw = t / nv;
@@ -606,7 +607,7 @@ int dga_chi0_prep_c128(const void* chi0, int n_orb, int niv_core, int niv_shell,
   const long long n_mats = (long long)n_q * niw_half * nv;
   const int th = small_threads(n2);
   const size_t smem = (size_t)th * n2 * n2 * sizeof(double2);
-  allow_shared_memory(chi0_inverse_kernel);
+  allow_shared_memory(chi0_inverse_kernel, smem);
   chi0_inverse_kernel<<<(int)((n_mats + th - 1) / th), th, smem, stream>>>(
       (const double2*)chi0, n2, nvf, nv, niv_shell, n_mats, (double2*)chi0_inv, status);
   if (vstatus("dga_chi0_prep_c128")) return DGA_ERR_LAUNCH;
@@ -647,7 +648,7 @@ int dga_lambda_c128(const void* chi, int n_q, int niw_half, int n_ch, const long
   }
   const long long per = ((long long)n_q * niw_half + LAMBDA_CTAS - 1) / LAMBDA_CTAS;
   const size_t smem = (size_t)(per < LAMBDA_CACHED ? per : LAMBDA_CACHED) * sizeof(double2);
-  allow_shared_memory(lambda_kernel);
+  allow_shared_memory(lambda_kernel, smem);
   lambda_kernel<<<n_ch * LAMBDA_CTAS, LAMBDA_THREADS, smem, stream>>>((const double2*)chi, n_q, niw_half, weights,
                                                                       (const double2*)target, beta, nk_tot, delta, eps,
                                                                       maxiter, lambda_out, iters_out, status,
@@ -669,7 +670,7 @@ int dga_kernel_assembly_c128(const void* chi0_inv, const void* X, const void* uv
   const int blocks = (int)((total + per_block - 1) / per_block);
 #define DGA_KA_CASE(NN)                                                                                        \
   case NN:                                                                                                     \
-    allow_shared_memory(kernel_assembly_kernel<NN>);                                                           \
+    allow_shared_memory(kernel_assembly_kernel<NN>, smem);                                                     \
     kernel_assembly_kernel<NN><<<blocks, 32 * KA_WARPS, smem, stream>>>(                                       \
         (const double2*)chi0_inv, (const double2*)X, (const double2*)uv, (const double2*)chi_phys,             \
         (const double2*)k_dc, 2 * niv_core, niw_half, n_q, beta, (double2*)K, (double2*)gamma_out);            \
@@ -712,7 +713,7 @@ int dga_dc_kernel_c128(const void* chi0, const void* u_perm, const void* fdc, in
     return DGA_ERR_ARG;
   }
   const size_t left_smem = (size_t)nus * ((n2 * n2) | 1) * sizeof(double2);
-  allow_shared_memory(dc_left_kernel);
+  allow_shared_memory(dc_left_kernel, left_smem);
   dc_left_kernel<<<(int)left_blocks, 256, left_smem, stream>>>(
       (const double2*)chi0, (const double2*)u_perm, n2, n_q, niw_half, nvf, nus, (double2*)scratch);
   if (vstatus("dga_dc_kernel_c128")) return DGA_ERR_LAUNCH;
