@@ -59,7 +59,6 @@ struct LuSmem {
   double2 us[8][NB];               // panel: rows of U of the columns just factored
   double2 cand[2][NT / 32][10];    // panel: each warp's candidate pivot row, conj(pivot), 1 / |pivot|^2
   __align__(16) unsigned long long key[2][(NT / 32 + 1) / 2 * 2];
-  int at[2][NT / 32];              // its position
   int flag;
 };
 
@@ -313,6 +312,8 @@ __device__ __forceinline__ unsigned long long lu_key(double2 a) {
   return x > LU_INF_BITS ? 0 : x + 1;
 }
 
+__device__ __forceinline__ int lu_cand_at(const double2* cand) { return __double2loint(cand[9].y); }
+
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long key) {
   const unsigned hi = (unsigned)(key >> 32);
   const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
@@ -454,25 +455,31 @@ __device__ bool lu_panel(double2* __restrict__ A, int N, int ld, int j0, int nb,
               for (int c = 0; c < PW; ++c) sm.cand[buf][warp][c] = a[i][c];
             }
           sm.cand[buf][warp][8] = rc;
-          sm.cand[buf][warp][9].x = rs;
-          sm.at[buf][warp] = at;
+          sm.cand[buf][warp][9] = make_double2(rs, __hiloint2double(0, at));
         }
         if (lane == 0) sm.key[buf][warp] = key;
         __syncthreads();
-        int p = sm.at[buf][0], win = 0;
+        int win = 0;
         if constexpr (NW > 1) {
-          key = sm.key[buf][0];
+          const ulonglong2* keys = reinterpret_cast<const ulonglong2*>(sm.key[buf]);
+          key = 0;
+          bool tie = false;
 #pragma unroll
-          for (int w = 1; w < NW; ++w) {
-            const unsigned long long x = sm.key[buf][w];
-            const int q = sm.at[buf][w];
-            if (x > key || (x == key && q < p)) {
-              key = x;
-              p = q;
-              win = w;
-            }
+          for (int w = 0; w < NW / 2; ++w) {
+            const ulonglong2 x = keys[w];
+            const unsigned long long m = x.x > x.y ? x.x : x.y;
+            const bool more = m > key;
+            tie = more ? x.x == x.y : tie || m == key;
+            win = more ? 2 * w + (x.y > x.x) : win;
+            key = more ? m : key;
+          }
+          if (tie && key) {
+#pragma unroll 1
+            for (int w = win + 1; w < NW; ++w)
+              if (sm.key[buf][w] == key && lu_cand_at(sm.cand[buf][w]) < lu_cand_at(sm.cand[buf][win])) win = w;
           }
         }
+        int p = lu_cand_at(sm.cand[buf][win]);
         if (key == 0) {  // no comparable entry (every one is NaN): the diagonal row stays
           p = j;
           win = 0;
