@@ -50,12 +50,15 @@ __global__ void __launch_bounds__(BSE_THREADS, 3)
   }
 }
 
-// out_m[:, k] = A_m^-1 B_m[:, k] for k < n_rhs, column-major with leading dimension N, DENSE_COLS
-// columns a CTA (columns n_rhs .. of the last 16 are solved for zero right-hand sides): substitution by 32-row blocks, each
-// accumulated on the FP64 tensor pipe over all solved blocks, with the diagonal blocks inverted.  B_m(r, k) =
+// out_m[:, k] = A_m^-1 B_m[:, k] for k < n_rhs, column-major with leading dimension N, COLS
+// columns a CTA (columns n_rhs .. of the last 16 are solved for zero right-hand sides): substitution by 32-row blocks.
+// DENSE_COLS: 16 columns a warp, each block accumulated on the FP64 tensor pipe over all solved blocks, with the diagonal
+// blocks inverted.  DENSE_RHS: 16 columns a CTA, whose threads split the rows under (over) each solved block
+// (dense_rows_form has the rule).  B_m(r, k) =
 // b[m b_sm + r b_sr + k b_sk], or the identity when b is null.  A non-finite solution element sets
 // DGA_ITEM_NONFINITE in status[m].
-__global__ void __launch_bounds__(BSE_THREADS, fp64_min_blocks(BSE_THREADS))
+template <int COLS>
+__global__ void __launch_bounds__(BSE_THREADS, COLS == DENSE_RHS ? 3 : fp64_min_blocks(BSE_THREADS))
     dense_solve_kernel(const double2* __restrict__ lu, const int* __restrict__ piv, int N, int n_mat,
                        long long lu_stride, const double2* __restrict__ b, long long b_sm, long long b_sr,
                        long long b_sk, int n_rhs, double2* __restrict__ out, long long out_stride,
@@ -64,9 +67,9 @@ __global__ void __launch_bounds__(BSE_THREADS, fp64_min_blocks(BSE_THREADS))
   Fp64Smem<BSE_THREADS>& sm = *reinterpret_cast<Fp64Smem<BSE_THREADS>*>(smem_raw);
   int* perm = reinterpret_cast<int*>(smem_raw + sizeof(Fp64Smem<BSE_THREADS>));
   const int tid = threadIdx.x, T = blockDim.x;
-  const int cols = (n_rhs + DENSE_RHS - 1) / DENSE_RHS * DENSE_RHS, n_blk = (cols + DENSE_COLS - 1) / DENSE_COLS;
+  const int cols = (n_rhs + DENSE_RHS - 1) / DENSE_RHS * DENSE_RHS, n_blk = (cols + COLS - 1) / COLS;
   for (int t = blockIdx.x; t < n_mat * n_blk; t += gridDim.x) {
-    const int m = t / n_blk, k0 = (t - m * n_blk) * DENSE_COLS, nc = min(DENSE_COLS, cols - k0);
+    const int m = t / n_blk, k0 = (t - m * n_blk) * COLS, nc = min(COLS, cols - k0);
     const int* pv = piv + (size_t)m * N;
     build_perm(N, pv, perm);
     double2* Y = out + (size_t)m * out_stride + (size_t)k0 * N;
@@ -84,8 +87,12 @@ __global__ void __launch_bounds__(BSE_THREADS, fp64_min_blocks(BSE_THREADS))
     }
     __syncthreads();
     const double2* f = lu + (size_t)m * lu_stride;
-    lu_forward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
-    lu_backward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
+    if constexpr (COLS == DENSE_RHS) {
+      lu_solve_inplace<double2, double2, DENSE_RHS>(f, N, N, Y, sm.solve.L11, sm.solve.yb);
+    } else {
+      lu_forward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
+      lu_backward_dmma<BSE_THREADS, 32>(f, N, N, Y, N, nc, sm.lu32);
+    }
     int bad = 0;
     for (int e = tid; e < N * nc; e += T) {
       const double2 v = Y[e];
@@ -979,6 +986,17 @@ int dga_lu_batched_c128(void* a, int N, int n_mat, long long mat_stride, int* pi
   return DGA_OK;
 }
 
+// Whether 16 columns get a CTA (true) or a warp. A warp's chain of products over the solved rows is the longer one from about
+// N = 400, as long as all CTAs of the first kind are resident at once, three an SM: 21 matrices of N = 720 with 64 columns
+// 2.5 against 3.7 ms, one with 720 columns 2.0 against 2.6, 82 with 96 columns (492 CTAs) 5.4 against 4.0; N = 400 with 64
+// columns 0.92 against 0.93, N = 320 0.69 against 0.61. With a single warp in each CTA and factors that do not stay in
+// L2, HBM's latency adds to the chain: 82 matrices with 16 columns 0.98 against 1.07 ms at N = 360, 0.81 either way at 320.
+static bool dense_rows_form(int N, int n_mat, long long cols) {
+  if (n_mat * (cols / DENSE_RHS) > 3LL * device_sm_count()) return false;
+  const bool from_hbm = cols == DENSE_RHS && (size_t)n_mat * N * N * sizeof(double2) > ((size_t)126 << 20);
+  return N > (from_hbm ? 320 : 400);
+}
+
 // Solves with the factors of dga_lu_batched_c128 for n_rhs right-hand sides (b null: the identity).
 int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, long long lu_stride, const void* b,
                               long long b_stride_m, long long b_stride_r, long long b_stride_k, int n_rhs, void* out,
@@ -990,15 +1008,23 @@ int dga_lu_solve_batched_c128(const void* lu, const int* piv, int N, int n_mat, 
     return DGA_ERR_ARG;
   }
   const size_t smem = sizeof(Fp64Smem<BSE_THREADS>) + sizeof(int) * (size_t)N;
-  const long long n_tasks = (long long)n_mat * ((cols + DENSE_COLS - 1) / DENSE_COLS);
+  const bool rows = dense_rows_form(N, n_mat, cols);
+  const int per_cta = rows ? DENSE_RHS : DENSE_COLS;
+  const long long n_tasks = (long long)n_mat * ((cols + per_cta - 1) / per_cta);
   if (n_tasks > 0x7fffffffLL) {
     dga_set_error("dga_lu_solve_batched_c128: too many right-hand-side blocks");
     return DGA_ERR_ARG;
   }
-  const int grid = grid_for(dense_solve_kernel, (int)n_tasks, smem);
-  dense_solve_kernel<<<grid, BSE_THREADS, smem, stream>>>((const double2*)lu, piv, N, n_mat, lu_stride,
-                                                          (const double2*)b, b_stride_m, b_stride_r, b_stride_k,
-                                                          n_rhs, (double2*)out, out_stride, status);
+  const auto go = [&](auto kernel) {
+    const int grid = grid_for(kernel, (int)n_tasks, smem);
+    kernel<<<grid, BSE_THREADS, smem, stream>>>((const double2*)lu, piv, N, n_mat, lu_stride, (const double2*)b,
+                                                b_stride_m, b_stride_r, b_stride_k, n_rhs, (double2*)out, out_stride,
+                                                status);
+  };
+  if (rows)
+    go(dense_solve_kernel<DENSE_RHS>);
+  else
+    go(dense_solve_kernel<DENSE_COLS>);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) {
     dga_set_error("dga_lu_solve_batched_c128: launch failed: %s", cudaGetErrorString(err));

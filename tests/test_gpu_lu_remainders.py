@@ -23,14 +23,16 @@ def _abs_lu(a):
     return p @ (np.abs(low) @ np.abs(up))
 
 
-# N % 32 = 1 .. 8, and 16, where no block is short
-@pytest.mark.parametrize("N", [33, 34, 35, 36, 37, 38, 39, 40, 65, 72, 200, 257, 16, 48])
-def test_dense_solve(N):
+# N % 32 = 1 .. 8, and 16, where no block is short; then both sides of the rule that gives 16 columns a CTA or a warp: N = 320
+# (factors beyond L2, 16 columns) and 400, three CTAs an SM
+@pytest.mark.parametrize("N,n,k", [(N, 300, N) for N in (33, 34, 35, 36, 37, 38, 39, 40, 65, 72, 200, 257, 16, 48)]
+                         + [(320, 82, 16), (321, 82, 16), (321, 82, 17), (400, 28, 240), (401, 28, 240), (401, 30, 240),
+                            (402, 1, 1), (416, 3, 33), (720, 21, 64), (1000, 1, 16)])
+def test_dense_solve(N, n, k):
     import torch
 
     from dgamore_b200._lib import call
 
-    n, k = 300, N
     cols = (k + 15) // 16 * 16
     g = torch.Generator(device="cuda").manual_seed(N)
     a = torch.randn((n, N, N), dtype=torch.complex128, device="cuda", generator=g)  # column-major: a[m].T
@@ -58,7 +60,7 @@ def test_dense_solve(N):
             perm[m, [i, q]] = perm[m, [q, i]]
     perm = torch.from_numpy(perm).cuda()[:, :, None].expand(-1, -1, N)
     # factorisation, two substitutions and the residual itself, N eps each (complex products: a factor of 8), rows in pivot order
-    res = torch.gather(mat, 1, perm) @ sol - torch.gather(eye.expand(n, N, N), 1, perm)
+    res = torch.gather(mat, 1, perm) @ sol - torch.gather(eye.expand(n, N, N), 1, perm)[:, :, :k]
     size = size + torch.gather(mat, 1, perm).abs()
     assert (res.abs() <= 8 * N * EPS * (size @ sol.abs()) + 8 * N * EPS).all()
 
