@@ -353,8 +353,9 @@ static size_t mixed_slot_bytes(int N, int n2) {
   return (((size_t)N * N * sizeof(float2) + 255) & ~(size_t)255) + 2 * (size_t)N * n2 * sizeof(double2);
 }
 // Default launch of the mixed form: the block-form kernel (4) wherever its solve phase fits shared memory (it is
-// the fastest at every size measured, N = 40 to 720); else, from N = 320, the shared-memory-panel kernel with
-// tensor-core trailing tiles (3) or FP32 tiles (1), else the 128-thread kernel (2).
+// the fastest of the mixed kernels at every size measured, N = 40 to 720; the FP64 form is the faster one for one orbital
+// at N = 40 and 120); else, from N = 320, the shared-memory-panel kernel with tensor-core trailing tiles (3) or FP32
+// tiles (1), else the 128-thread kernel (2).
 static int default_mixed_kernel(int N, int n2) {
   if (dga_block_supported(N, n2)) return 4;
   if (N < 320) return 2;

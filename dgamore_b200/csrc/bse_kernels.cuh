@@ -1037,12 +1037,12 @@ __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))
 
 // ----------------------------------------------------------------------------------------------
 // Dense batched LU and solves with many right-hand sides (the local Schwinger-Dyson equation's full inverses,
-// numpy.linalg.inv behind LocalFourPoint.invert, local_four_point.py:298-310).  The factorisation is lu_factor
-// (LAPACK's pivot order) with one CTA per matrix; the solves spread over (matrix, block of DENSE_RHS right-hand
-// sides) CTAs, each streaming the factors once for its block.
+// numpy.linalg.inv behind LocalFourPoint.invert, local_four_point.py:298-310).  The factorisation is lu_factor_dmma
+// (LAPACK's pivot order) with one CTA per matrix, lu_factor beyond N = 2048; the solves spread over (matrix, block of
+// DENSE_COLS or DENSE_RHS right-hand sides) CTAs, each streaming the factors once for its block.
 // ----------------------------------------------------------------------------------------------
-constexpr int DENSE_RHS = 16;   // right-hand sides are padded to a multiple of this
-constexpr int DENSE_COLS = 64;  // columns a CTA solves: 16 a warp
+constexpr int DENSE_RHS = 16;   // right-hand sides are padded to a multiple of this; columns a CTA solves by rows
+constexpr int DENSE_COLS = 64;  // columns a CTA solves with 16 a warp
 
 template <int NT>
 __global__ void __launch_bounds__(NT, fp64_min_blocks(NT))

@@ -7,14 +7,15 @@
 // Why Crout order: a right-looking update reads and writes the whole trailing matrix once per 32 columns (2/3 N^3 / 32
 // elements read and written, 248 MB at N = 720 with the factor tiles); here a block column and a block row are
 // accumulated in registers over everything to their left and above and written once, so the same products cost
-// reads only (62 MB at N = 720), and a CTA needs no shared-memory tiles or barriers inside them.
+// reads only (62 MB by count at N = 720; a whole item of the BSE moves 123 MB of DRAM, 173 before), and a CTA needs no
+// shared-memory tiles or barriers inside them.
 //
 // Why mma.sync f64: the FP64 tensor pipe and the FP64 vector pipe have the same peak (37 TFLOP/s measured for either),
 // but an m16n8k4 product takes one warp instruction where the vector pipe takes 16, and its A and B fragments of an
 // interleaved complex matrix are one 16-byte load per lane each (lane (g, t) holds row g and column t), so operands come
 // straight from L2 and L1: four warps per SM already reach 35 TFLOP/s. The tcgen05 pipe has no FP64 kind.
 //
-// What bounds it: the products at N = 720 (592 factorisations in 27.9 ms, 21.1 TFLOP/s, two CTAs an SM), waits on HBM and
+// What bounds it: the products at N = 720 (592 factorisations in 28.1 ms, 21.0 TFLOP/s, two CTAs an SM), waits on HBM and
 // L2 for the panels and the tiles' first elements below about N = 250 (14,208 of N = 120 in 6.8 ms, 9.6 TFLOP/s).
 #pragma once
 
@@ -114,8 +115,8 @@ __device__ __forceinline__ void cdmma_row(CAcc* c, double2 a0, double2 a1, const
 }
 
 // Block column: A[j0.., j0 .. j0+nb) -= A[j0.., 0..j0) A[0..j0, j0 .. j0+nb). One warp per 16 rows x NB columns; rows and
-// columns past the end read the last valid ones and are not stored. L streams from HBM (the matrices in flight are ten
-// times L2): a lane copies the two elements it multiplies three steps later, 1,500 cycles of the FP64 pipe at NB = 32, into its own
+// columns past the end read the last valid ones and are not stored. L streams from HBM (the matrices in flight are twice
+// L2 at N = 120 and twenty times at N = 720): a lane copies the two elements it multiplies three steps later, 1,500 cycles of the FP64 pipe at NB = 32, into its own
 // ring slot, so nothing has to be synchronised; U is shared by all warps and comes from L1, one step ahead.
 template <int NT, int NB>
 __device__ void lu_block_column(double2* __restrict__ A, int N, int ld, int j0, int nb, LuSmem<NT, NB>& sm) {
@@ -646,9 +647,10 @@ __device__ void lu_invert_upper(const double2* __restrict__ A, int ld, int j0, i
   __syncthreads();
 }
 
-// The block's row interchanges on the columns outside it: in parallel over (interchange, column) when they are
-// independent pairs (every pivot row below the block, no two alike), else in order per column; nothing to do when no
-// row moved.
+// The block's row interchanges on the columns outside it, a thread per column: one interchange after the other over all
+// columns when they are independent pairs (every pivot row below the block, no two alike), else all of a column's in turn;
+// nothing to do when no row moved. (One loop in order for every case: 3,552 of N = 240 whose rows all move take 15.8 ms
+// instead of 14.9; a thread per pair and column, four in flight: 82 of N = 720 13.6 instead of 12.9.)
 template <int NT, int NB>
 __device__ void lu_interchange(double2* __restrict__ A, int ncols, int ld, int j0, int nb, const int* __restrict__ piv,
                                LuSmem<NT, NB>& sm) {

@@ -197,27 +197,9 @@ chi_phys_kernel(const double2* __restrict__ X, const double2* __restrict__ uv, c
 }
 
 // ------------------------------------------------------------------------------------------------
-// lambda correction (single band): one CTA per channel
+// lambda correction (single band)
 //   chi: [n_ch][Q][W] (n2 = 1), weights = irrk_count, target[ch] complex
 // ------------------------------------------------------------------------------------------------
-__device__ double block_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    v = lane < nw ? red[lane] : 0.0;
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) red[0] = v;
-  }
-  __syncthreads();
-  const double r = red[0];
-  __syncthreads();
-  return r;
-}
-
 __device__ double block_min(double v, double* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int off = 16; off > 0; off >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, off));
